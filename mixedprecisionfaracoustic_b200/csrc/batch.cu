@@ -63,7 +63,7 @@ int BatchCore::rebuild() {
         h[i].tile0f = t0f;
         h[i].item0_i = t0i;
         h[i].band0_i = nbands;
-        t0i += apply_bands(h[i], dim, tiles, ctas_i);
+        t0i += apply_bands(h[i], dim, ctas_i);
         nbands += h[i].nbands_i;
         h[i].done = 0;
         t0f += shots[i]->ntiles_f;

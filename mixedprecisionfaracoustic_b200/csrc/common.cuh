@@ -60,6 +60,12 @@ struct ShotDesc {
     // 2^(tile_lr - tile_ltz) y rows of 2^tile_ltz z planes) x 2^tile_ls
     // 128-cell segments; nseg_t = tiles per row block along x
     int tile_lr, tile_ls, tile_ltz, nseg_t;
+    // flat tiling of the register kernels: cpr 4-cell chunks per row, nyb row
+    // blocks per z block (3D), nchunk_f chunks in all row blocks; n / cpr =
+    // n * cpr_m >> cpr_s, likewise nyb
+    int cpr, cpr_s, nyb, nyb_s;
+    unsigned cpr_m, nyb_m;
+    int nchunk_f, pad_fl;
     int nt;                       // trace length
     int src_idx_valid;
     long long src_idx;            // flat index of the source cell

@@ -513,7 +513,7 @@ int Shot::create(const bp_config* c, const bp_medium* med, cudaStream_t st) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         S.item0_i = 0;
         S.band0_i = 0;
-        nitems_i = apply_bands(S, dim, ntiles, inter_occupancy(c->precision, dim, c->order, c->rounding) * sms);
+        nitems_i = apply_bands(S, dim, inter_occupancy(c->precision, dim, c->order, c->rounding) * sms);
     }
     d_desc = (ShotDesc*)(A + p.o_desc);
     if (e == cudaSuccess)

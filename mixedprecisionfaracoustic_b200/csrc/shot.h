@@ -44,7 +44,7 @@ long long apply_tile_shape(ShotDesc& S, int dim, int prec, TileShape t);
 // Groups the shot's tiles (current shape, ntiles of them) into the bands of
 // the interleaved step kernel, for a launch of `ctas` persistent CTAs; returns
 // the shot's work items (2 x ntiles).
-long long apply_bands(ShotDesc& S, int dim, long long ntiles, int ctas);
+long long apply_bands(ShotDesc& S, int dim, int ctas);
 // indexed medium (medium_index.cu): *ntuples = 0 leaves the shot on its arrays
 size_t medium_scratch_bytes();
 void algorithmic_bpc(const bp_config& c, bool indexed, double bpc[2]);   // sim.cu

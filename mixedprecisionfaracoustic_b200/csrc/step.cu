@@ -10,8 +10,9 @@
 //
 // Work decomposition: a tile is 8 rows x 128 cells of one shot; a CTA of 8
 // warps takes one tile at a time (one row per warp, 4 consecutive x cells per
-// lane, 16-byte vector accesses along x).  CTAs loop over the tile table of
-// all shots of a batch, so one launch advances every shot by one phase.
+// lane, 16-byte vector accesses along x; the 128 cells run on into the next
+// row block where a row ends, flat_cell in tile.cuh).  CTAs loop over the tile
+// table of all shots of a batch, so one launch advances every shot by one phase.
 // Neighbour rows (y, z) are re-read through L1/L2; DRAM sees each array once
 // per phase.  The CPML memory variables exist on the slabs only; a chunk
 // touches them only when it lies in a slab of that axis.
@@ -51,23 +52,15 @@ __global__ void __launch_bounds__(kThreads, (phase_min_blocks<DIM, ORD, P, VPHAS
             }
         }
         const ShotDesc& S = sdesc;
-        int rb, sb;                           // row block and segment block of the tile
         if constexpr (step_once_per_shot<P>()) {
             if (!live) continue;
-            const unsigned lt = (unsigned)(t - S.tile0);      // tiles of one shot < 2^32
-            const unsigned q = lt / (unsigned)S.nseg_t;
-            rb = (int)q;
-            sb = (int)(lt - q * (unsigned)S.nseg_t);
         } else {
             const int it = *S.step_base + k;
             if (S.done || it >= S.nt) continue;
             it_cur = it;
             if constexpr (P::prec == BP_PREC_COMP16) r = S.rtab[it];
-            const long long lt = t - S.tile0;
-            rb = (int)(lt / S.nseg_t);
-            sb = (int)(lt % S.nseg_t);
         }
-        tile_units<DIM, ORD, P, VPHASE, MU, true>(S, rb, sb, warp, lane, r, it_cur, post);
+        flat_units<DIM, ORD, P, VPHASE, MU, true>(S, (int)(t - S.tile0), warp, lane, r, it_cur, post);
     }
 }
 
@@ -320,6 +313,31 @@ static int ilog2(int v) {
 }
 static bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
+// Chunks per row of the flat tiling, n for a row without gaps.  Rows that start
+// on 64-byte boundaries of the field arrays (FP32: 128-byte lines where that
+// adds at most 6 % of empty chunks) keep a warp's pieces of two rows from
+// sharing the memory's fetch unit with other warps: 296 x 296 x 232 with a
+// per-cell medium reads 3.03 GB in the V phase without gaps, 2.57 GB with 80
+// chunks for 74, and takes 1435 -> 1190 (76) or 1267 (80) us per step; CBF16
+// there 1690 -> 1374 (80).  Gaps above 9 % cost more than they save (CBF16 140
+// x 130 x 120, 35 chunks: 208 us without, 228 at 40).  COMP16, bound by its
+// codec's instructions, takes no gaps (140 x 130 x 120: 233 against 296 us).
+static int row_chunks(int n, int prec) {
+    const int a64 = prec == BP_PREC_FP64 ? 2 : prec == BP_PREC_FP32 ? 4 : 8;
+    auto up = [&](int a) { return (n + a - 1) / a * a; };
+    if (prec == BP_PREC_FP32 && (up(2 * a64) - n) * 100 <= 6 * n) return up(2 * a64);
+    if (prec != BP_PREC_COMP16 && (up(a64) - n) * 100 <= 9 * n) return up(a64);
+    return n;
+}
+
+// Reciprocal of d >= 1 for div_magic: p = 31 + ceil(log2 d), m = ceil(2^p / d)
+// < 2^32, and n m >> p = n / d for every 0 <= n < 2^31.
+static void magic_of(int d, unsigned& m, int& s) {
+    s = 31;
+    while ((1LL << (s - 31)) < d) s++;
+    m = (unsigned)(((1ULL << s) + d - 1) / d);
+}
+
 TileShape default_tile_shape(int dim, int prec) {
     TileShape t;
     t.rows = kWarps;
@@ -341,14 +359,14 @@ long long apply_tile_shape(ShotDesc& S, int dim, int prec, TileShape t) {
     S.tile_ls = ilog2(t.segs);
     S.tile_ltz = ilog2(t.tz);
     S.nseg_t = (S.nseg + t.segs - 1) / t.segs;
-    long long blocks;
-    if (dim == 3) {
-        const int ty = t.rows / t.tz;
-        blocks = (long long)((S.ny + ty - 1) / ty) * ((S.nz + t.tz - 1) / t.tz);
-    } else {
-        blocks = (S.nrows + t.rows - 1) / t.rows;
-    }
-    return blocks * S.nseg_t;
+    const int ty = dim == 3 ? t.rows / t.tz : 1;
+    S.nyb = dim == 3 ? (S.ny + ty - 1) / ty : 1;
+    const long long blocks = dim == 3 ? (long long)S.nyb * ((S.nz + t.tz - 1) / t.tz) : (S.nrows + t.rows - 1) / t.rows;
+    S.cpr = row_chunks((S.nx + 3) / 4, prec);
+    magic_of(S.cpr, S.cpr_m, S.cpr_s);
+    magic_of(S.nyb, S.nyb_m, S.nyb_s);
+    S.nchunk_f = (int)(blocks * S.cpr);
+    return (blocks * S.cpr + 32LL * t.segs - 1) / (32LL * t.segs);
 }
 int seg_cells() { return kSegCells; }
 }  // namespace bpk

@@ -188,18 +188,22 @@ __global__ void __launch_bounds__(kThreads, (inter_min_blocks<DIM, ORD, P>())) k
 // ---------------------------------------------------------------------------
 bool inter_default() { return BP_INTER_DEFAULT != 0; }
 
-long long apply_bands(ShotDesc& S, int dim, long long ntiles, int ctas) {
+long long apply_bands(ShotDesc& S, int dim, int ctas) {
     int rb_per_band;
+    long long blocks;
     if (dim == 3) {
         const int lty = S.tile_lr - S.tile_ltz;
         const int nyb = (S.ny + (1 << lty) - 1) >> lty;
         const int tz = 1 << S.tile_ltz;
         const int bz = (BP_INTER_BAND_PLANES + tz - 1) / tz;
         rb_per_band = bz * nyb;
+        blocks = (long long)nyb * ((S.nz + tz - 1) / tz);
     } else {
         const int rows = 1 << S.tile_lr;
         rb_per_band = (BP_INTER_BAND_ROWS + rows - 1) / rows;
+        blocks = (S.nrows + rows - 1) / rows;
     }
+    const long long ntiles = blocks * S.nseg_t;
     const long long tpb = (long long)rb_per_band * S.nseg_t;
     const int nb = (int)((ntiles + tpb - 1) / tpb);
     S.band_t = (int)tpb;

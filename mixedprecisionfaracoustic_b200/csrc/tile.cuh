@@ -655,17 +655,52 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int 
 }
 
 // ---------------------------------------------------------------------------
-// The (row, segment) units of tile (rb, sb) of shot S in one phase (it: the
-// step index, r: the COMP16 rescale factor of that step).  post (T phase
-// only): each chunk also records the receivers in its cells and, if it holds
-// the source cell, injects the next source sample, in place of the post-step
-// kernel k_post.
+// One chunk of one phase: cells x0 .. x0 + 3 of row (y, z) (it: the step index,
+// r: the COMP16 rescale factor of that step), nothing if the phase updates none
+// of them.  post (T phase only): the chunk also records the receivers in its
+// cells and, if it holds the source cell, injects the next source sample, in
+// place of the post-step kernel k_post.
+template <int DIM, int ORD, class P, bool VPHASE, bool NCOK>
+__device__ __forceinline__ void chunk_unit(const ShotDesc& S, int x0, int y, int z, typename P::real r, int it,
+                                           int post) {
+    using R = typename P::real;
+    const int hw = ORD / 2;
+    if (z < hw || z >= S.nz - hw) return;
+    if (DIM == 3 && (y < hw || y >= S.ny - hw)) return;
+    if (x0 >= S.nx - hw || x0 + 3 < hw) return;
+    unsigned mask = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (x0 + j >= hw && x0 + j < S.nx - hw) mask |= 1u << j;
+    // COMP16: the rescale products only on the steps whose factor is not
+    // exactly 1 (a uniform branch; the products are never fused, so both
+    // forms give the same bits when r == 1)
+    if constexpr (grouped<DIM, P, VPHASE>()) {
+        if (P::prec == BP_PREC_COMP16 && (r != (R)1 || !BP_RS_SPLIT)) {
+            if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, P::prec == BP_PREC_COMP16>(S, x0, y, z, r, mask);
+            else t_chunk_g<DIM, ORD, P, P::prec == BP_PREC_COMP16>(S, x0, y, z, r, mask);
+        } else {
+            if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, false>(S, x0, y, z, r, mask);
+            else t_chunk_g<DIM, ORD, P, false>(S, x0, y, z, r, mask);
+        }
+    } else if (P::prec == BP_PREC_COMP16 && (r != (R)1 || !BP_RS_SPLIT)) {
+        if constexpr (VPHASE) v_chunk<DIM, ORD, P, P::prec == BP_PREC_COMP16, NCOK>(S, x0, y, z, r, mask);
+        else t_chunk<DIM, ORD, P, P::prec == BP_PREC_COMP16, NCOK>(S, x0, y, z, r, mask);
+    } else {
+        if constexpr (VPHASE) v_chunk<DIM, ORD, P, false, NCOK>(S, x0, y, z, r, mask);
+        else t_chunk<DIM, ORD, P, false, NCOK>(S, x0, y, z, r, mask);
+    }
+    if constexpr (!VPHASE)
+        if (post) post_chunk<DIM, P>(S, it, x0 + y * (cidx)S.pitch + z * (cidx)S.plane, x0, y, z);
+}
+
+// The (row, segment) units of tile (rb, sb) of shot S in one phase: the
+// rectangular tiling of the interleaved step kernel, whose bands are whole row
+// blocks.  Warp w takes units w, w + 8, ...; consecutive warps take
+// consecutive rows.
 template <int DIM, int ORD, class P, bool VPHASE, bool MU, bool NCOK>
 __device__ __forceinline__ void tile_units(const ShotDesc& S, int rb, int sb, int warp, int lane, typename P::real r,
                                            int it, int post) {
-    using R = typename P::real;
-    // the tile's (row, segment) units, warp w taking units w, w + 8, ...;
-    // consecutive warps take consecutive rows
     const int lr = S.tile_lr, units = 1 << (lr + S.tile_ls);
     auto unit = [&](int u) {
         const int ri = u & ((1 << lr) - 1);
@@ -678,46 +713,69 @@ __device__ __forceinline__ void tile_units(const ShotDesc& S, int rb, int sb, in
             const int zb = rb / nyb, yb = rb - zb * nyb;
             y = (yb << lty) + (ri & ((1 << lty) - 1));
             z = (zb << ltz) + (ri >> lty);
-            if (y >= S.ny || z >= S.nz) return;
+            if (y >= S.ny) return;
         } else {
-            const int row = (rb << lr) + ri;
-            if (row >= S.nrows) return;
             y = 0;
-            z = row;
+            z = (rb << lr) + ri;
         }
-        const int hw = ORD / 2;
-        if (z < hw || z >= S.nz - hw) return;
-        if (DIM == 3 && (y < hw || y >= S.ny - hw)) return;
-        const int x0 = seg * kSegCells + lane * 4;
-        if (x0 >= S.nx - hw || x0 + 3 < hw) return;
-        unsigned mask = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (x0 + j >= hw && x0 + j < S.nx - hw) mask |= 1u << j;
-        // COMP16: the rescale products only on the steps whose factor is not
-        // exactly 1 (a uniform branch; the products are never fused, so both
-        // forms give the same bits when r == 1)
-        if constexpr (grouped<DIM, P, VPHASE>()) {
-            if (P::prec == BP_PREC_COMP16 && (r != (R)1 || !BP_RS_SPLIT)) {
-                if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, P::prec == BP_PREC_COMP16>(S, x0, y, z, r, mask);
-                else t_chunk_g<DIM, ORD, P, P::prec == BP_PREC_COMP16>(S, x0, y, z, r, mask);
-            } else {
-                if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, false>(S, x0, y, z, r, mask);
-                else t_chunk_g<DIM, ORD, P, false>(S, x0, y, z, r, mask);
-            }
-        } else if (P::prec == BP_PREC_COMP16 && (r != (R)1 || !BP_RS_SPLIT)) {
-            if constexpr (VPHASE) v_chunk<DIM, ORD, P, P::prec == BP_PREC_COMP16, NCOK>(S, x0, y, z, r, mask);
-            else t_chunk<DIM, ORD, P, P::prec == BP_PREC_COMP16, NCOK>(S, x0, y, z, r, mask);
-        } else {
-            if constexpr (VPHASE) v_chunk<DIM, ORD, P, false, NCOK>(S, x0, y, z, r, mask);
-            else t_chunk<DIM, ORD, P, false, NCOK>(S, x0, y, z, r, mask);
-        }
-        if constexpr (!VPHASE)
-            if (post) post_chunk<DIM, P>(S, it, x0 + y * (cidx)S.pitch + z * (cidx)S.plane, x0, y, z);
+        chunk_unit<DIM, ORD, P, VPHASE, NCOK>(S, seg * kSegCells + lane * 4, y, z, r, it, post);
     };
     // MU: tiles of more units than warps (16-row or 8 x 2 tiles); the
     // one-unit form keeps no loop state live across the chunk code, which
     // costs the 2D FP32 V phase its spill-free 80 registers otherwise
+    if constexpr (MU) {
+        for (int u = warp; u < units; u += kWarps) unit(u);
+    } else {
+        if (warp < units) unit(warp);
+    }
+}
+
+// n / d for 0 <= n < 2^31 by a product with the divisor's reciprocal
+// (magic_of): exact for every such n.
+__device__ __forceinline__ int div_magic(int n, unsigned m, int s) {
+    return (int)(((unsigned long long)(unsigned)n * m) >> s);
+}
+
+// Cell of chunk q of the flat tiling (row ri of its row block), false past the
+// shot's chunks.  The chunks of the row blocks follow each other, cpr of them a
+// row (row_chunks, step.cu), and a warp takes 32 consecutive ones: its lanes are
+// full where a row is no multiple of 128 cells.  Measured on B200 against rows
+// cut into 128-cell segments, whose last segment is 8-86 % empty (FP32, us per
+// step, segments -> flat): 200^3 order 2 544 -> 465, order 4 591 -> 515; 424 x
+// 424 x 328 per-cell medium 4408 -> 3390; 817 x 1073 23.7 -> 20.6; 192^3
+// reference rounding 746 -> 626; FP64 1040 x 540 56.5 -> 41.7; 4040 x 2040
+// (1 % empty) unchanged.  The kernels wait on loads, so a warp's work counts
+// whether its lanes are full or not.
+template <int DIM>
+__device__ __forceinline__ bool flat_cell(const ShotDesc& S, int q, int ri, int& x0, int& y, int& z) {
+    if (q >= S.nchunk_f) return false;
+    const int blk = div_magic(q, S.cpr_m, S.cpr_s);
+    x0 = (q - blk * S.cpr) * 4;
+    if constexpr (DIM == 3) {
+        const int ltz = S.tile_ltz, lty = S.tile_lr - ltz;
+        const int zb = div_magic(blk, S.nyb_m, S.nyb_s);
+        y = ((blk - zb * S.nyb) << lty) + (ri & ((1 << lty) - 1));
+        z = (zb << ltz) + (ri >> lty);
+        return y < S.ny && z < S.nz;
+    } else {
+        y = 0;
+        z = (blk << S.tile_lr) + ri;
+        return z < S.nz;
+    }
+}
+
+// The units of tile lt of shot S in the flat tiling.
+template <int DIM, int ORD, class P, bool VPHASE, bool MU, bool NCOK>
+__device__ __forceinline__ void flat_units(const ShotDesc& S, int lt, int warp, int lane, typename P::real r, int it,
+                                           int post) {
+    const int lr = S.tile_lr, units = 1 << (lr + S.tile_ls);
+    auto unit = [&](int u) {
+        const int ri = u & ((1 << lr) - 1);
+        const int q = (((lt << S.tile_ls) + (u >> lr)) << 5) + lane;
+        int x0, y, z;
+        if (!flat_cell<DIM>(S, q, ri, x0, y, z)) return;
+        chunk_unit<DIM, ORD, P, VPHASE, NCOK>(S, x0, y, z, r, it, post);
+    };
     if constexpr (MU) {
         for (int u = warp; u < units; u += kWarps) unit(u);
     } else {
