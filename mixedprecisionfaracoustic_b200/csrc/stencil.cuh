@@ -202,6 +202,40 @@ __device__ __forceinline__ void cpml_slot(R (&d)[4], void* base, long long cells
     }
 }
 
+// The memory variables of every slot of one axis at once (slot k: derivative
+// d[k], the half-grid profile if half bit k): all the loads before the first
+// store, so a chunk waits once for an axis instead of once per slot (the
+// compiler cannot move a load over a store to the same type).  Measured on B200,
+// us per step, slot by slot -> at once (FP32 where not named): 296 x 296 x 232
+// 1740 -> 1553, 4040 x 2040 179 -> 166, 817 x 1073 21.2 -> 19.3, 200^3 order 2
+// 492 -> 482; FP64 1040 x 540 40.0 -> 38.1.
+template <int NS, bool RS, class R, bool EX = false>
+__device__ __forceinline__ void cpml_axis(R (*const (&d)[NS])[4], unsigned half, void* base, long long cells,
+                                          cidx sidx, bool xaxis, int pos, int x0, const void* pb, const void* pe,
+                                          const void* pb2, const void* pe2, R r, void* out, bool st) {
+    R ps[NS][4], pv[NS][4];
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+        PsiIO<R>::ld(static_cast<const R*>(base) + (long long)k * cells + sidx, ps[k]);
+        PsiIO<R>::ld(static_cast<const R*>(base) + (long long)(NS + k) * cells + sidx, pv[k]);
+    }
+    R* o = static_cast<R*>(out ? out : base);
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+        const R* b = static_cast<const R*>((half >> k & 1) ? pb2 : pb);
+        const R* e = static_cast<const R*>((half >> k & 1) ? pe2 : pe);
+        if (xaxis) cpml_x<RS, R, EX>(*d[k], ps[k], pv[k], b, e, x0, r);
+        else cpml_s<RS, R, EX>(*d[k], ps[k], pv[k], b[pos], e[pos], r);
+    }
+    if (st) {
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            PsiIO<R>::st(o + (long long)k * cells + sidx, ps[k]);
+            PsiIO<R>::st(o + (long long)(NS + k) * cells + sidx, pv[k]);
+        }
+    }
+}
+
 // Slab memory-variable index of a chunk for one axis, or -1 outside the slab.
 __device__ __forceinline__ cidx slab_index(const ShotDesc& S, int axis, int x0, int y, int z) {
     const Slab& sl = S.slab[axis];
@@ -257,30 +291,49 @@ __device__ __forceinline__ void med_comp4(const ShotDesc& S, unsigned ids, int g
 #pragma unroll
     for (int j = 0; j < 4; j++) o[j] = (R)(q == 0 ? t[j].x : q == 1 ? t[j].y : q == 2 ? t[j].z : t[j].w);
 }
-// One V-phase coefficient (VCoef k) of the chunk at c.
+// One V-phase coefficient (VCoef k) of the chunk at c (ids: its tuple indices).
 template <class P, bool NC = kReadOnlyPath>
-__device__ __forceinline__ void vcoef4(const ShotDesc& S, int k, cidx c, typename P::real (&o)[4]) {
+__device__ __forceinline__ void vcoef4(const ShotDesc& S, int k, cidx c, unsigned ids, typename P::real (&o)[4]) {
     if (med_on<P>(S)) {
         const int g = (k == VC_RHO_Y || k == VC_CC1_Y || k == VC_CC2_Y) ? MED_V_Y
                       : (k == VC_RHO_Z || k == VC_CC1_Z || k == VC_CC2_Z) ? MED_V_Z : MED_V_X;
         const int q = k == VC_RHOF ? 3 : (k == VC_RHO_X || k == VC_RHO_Y || k == VC_RHO_Z) ? 0
                       : (k == VC_CC1_X || k == VC_CC1_Y || k == VC_CC1_Z) ? 1 : 2;
-        med_comp4(S, med_ids(S, c), g, q, o);
+        med_comp4(S, ids, g, q, o);
         return;
     }
     P::template ld4<NC>(S.vc[k], S.vclo[k], c, o);
 }
 // One T-phase coefficient (TCoef k) of the chunk at c.
 template <class P, bool NC = kReadOnlyPath>
-__device__ __forceinline__ void tcoef4(const ShotDesc& S, int k, cidx c, typename P::real (&o)[4]) {
+__device__ __forceinline__ void tcoef4(const ShotDesc& S, int k, cidx c, unsigned ids, typename P::real (&o)[4]) {
     if (med_on<P>(S)) {
         const int g = (k == TC_C || k == TC_M || k == TC_H || k == TC_H2U) ? MED_T_A : MED_T_B;
         const int q = (k == TC_C || k == TC_MUXZ) ? 0 : (k == TC_M || k == TC_MUXY) ? 1
                       : (k == TC_H || k == TC_MUYZ) ? 2 : 3;
-        med_comp4(S, med_ids(S, c), g, q, o);
+        med_comp4(S, ids, g, q, o);
         return;
     }
     P::template ld4<NC>(S.tc[k], S.tclo[k], c, o);
+}
+
+// The chunk's old values of a field the phase updates, from its array.
+template <class P>
+struct ArraySrc {
+    const ShotDesc& S;
+    cidx c;
+    template <int F>
+    __device__ __forceinline__ void own(typename P::real (&v)[4]) const { P::ld4(S.f[F], S.flo[F], c, v); }
+};
+
+// The same with the tuple indices loaded here.
+template <class P, bool NC = kReadOnlyPath>
+__device__ __forceinline__ void vcoef4(const ShotDesc& S, int k, cidx c, typename P::real (&o)[4]) {
+    vcoef4<P, NC>(S, k, c, med_on<P>(S) ? med_ids(S, c) : 0u, o);
+}
+template <class P, bool NC = kReadOnlyPath>
+__device__ __forceinline__ void tcoef4(const ShotDesc& S, int k, cidx c, typename P::real (&o)[4]) {
+    tcoef4<P, NC>(S, k, c, med_on<P>(S) ? med_ids(S, c) : 0u, o);
 }
 
 template <class R>
@@ -294,9 +347,9 @@ struct VState {
 
 // On return V's old-velocity members (vu_*, vw_*) hold the new velocities as a
 // later load of the stored values returns them.
-template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
+template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath, class Src>
 __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
-                                       unsigned mask, VState<typename P::real>& V, const TailOut& O) {
+                                       unsigned mask, VState<typename P::real>& V, const TailOut& O, const Src& src) {
     using R = typename P::real;
     auto &x1 = V.x1, &x3 = V.x3, &s1 = V.s1, &z1 = V.z1, &z2 = V.z2, &s3 = V.s3;
     auto &x2 = V.x2, &y1 = V.y1, &y2 = V.y2, &y3 = V.y3, &s2 = V.s2, &z3 = V.z3;
@@ -304,8 +357,7 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
     auto &rho_z = V.rho_z, &c1_z = V.c1_z, &c2_z = V.c2_z, &vu_z = V.vu_z, &vw_z = V.vw_z;
     auto &rho_y = V.rho_y, &c1_y = V.c1_y, &c2_y = V.c2_y, &vu_y = V.vu_y, &vw_y = V.vw_y;
     const bool med = med_on<P>(S);
-    auto load_axis = [&](int fu, int fw, int crho, int ccc1, int ccc2, R (&rho)[4], R (&c1)[4], R (&c2)[4],
-                         R (&vu)[4], R (&vw)[4]) {
+    auto load_axis = [&](int crho, int ccc1, int ccc2, R (&rho)[4], R (&c1)[4], R (&c2)[4]) {
         if (med) {
             // one group per cell: (rho, cc1, cc2, rhof) of this axis
             const int g = crho == VC_RHO_X ? MED_V_X : crho == VC_RHO_Y ? MED_V_Y : MED_V_Z;
@@ -321,8 +373,6 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
             P::template ld4<NC>(S.vc[ccc1], S.vclo[ccc1], c, c1);
             P::template ld4<NC>(S.vc[ccc2], S.vclo[ccc2], c, c2);
         }
-        P::ld4(S.f[fu], S.flo[fu], c, vu);
-        P::ld4(S.f[fw], S.flo[fw], c, vw);
     };
     // the rescale factor applies to old stresses: scale their derivatives
     if constexpr (P::prec == BP_PREC_COMP16 && RS) {
@@ -340,37 +390,25 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
     // ---- CPML memory variables on the slabs (Float/main.cu:130-158) ----
     {
         constexpr int NS = DIM == 3 ? 4 : 3;
-        cidx si = slab_index(S, 0, x0, y, z);
-        if (si >= 0) {
-            void* B = O.psi_in[0];
-            void* Bo = O.psi_out ? O.psi_out[0] : nullptr;
-            const long long n = S.slab_cells[0];
-            cpml_slot<NS, RS, R, P::exact>(x1, B, n, 0, si, true, x0, x0, S.pb2[0], S.pe2[0], r, Bo, O.store);
-            cpml_slot<NS, RS, R, P::exact>(s1, B, n, 1, si, true, x0, x0, S.pb2[0], S.pe2[0], r, Bo, O.store);
-            cpml_slot<NS, RS, R, P::exact>(z2, B, n, 2, si, true, x0, x0, S.pb[0], S.pe[0], r, Bo, O.store);
-            if constexpr (DIM == 3) cpml_slot<NS, RS, R, P::exact>(y2, B, n, 3, si, true, x0, x0, S.pb[0], S.pe[0], r, Bo, O.store);
-        }
+        // half-grid profile for the forward differences (bits by slot)
+        auto axis = [&](R (*const (&d)[NS])[4], unsigned half, int a, int pos) {
+            const cidx si = slab_index(S, a, x0, y, z);
+            if (si >= 0)
+                cpml_axis<NS, RS, R, P::exact>(d, half, O.psi_in[a], S.slab_cells[a], si, a == 0, pos, x0, S.pb[a],
+                                               S.pe[a], S.pb2[a], S.pe2[a], r, O.psi_out ? O.psi_out[a] : nullptr, O.store);
+        };
         if constexpr (DIM == 3) {
-            si = slab_index(S, 1, x0, y, z);
-            if (si >= 0) {
-                void* B = O.psi_in[1];
-                void* Bo = O.psi_out ? O.psi_out[1] : nullptr;
-                const long long n = S.slab_cells[1];
-                cpml_slot<NS, RS, R, P::exact>(x2, B, n, 0, si, false, y, x0, S.pb[1], S.pe[1], r, Bo, O.store);
-                cpml_slot<NS, RS, R, P::exact>(y1, B, n, 1, si, false, y, x0, S.pb2[1], S.pe2[1], r, Bo, O.store);
-                cpml_slot<NS, RS, R, P::exact>(s2, B, n, 2, si, false, y, x0, S.pb2[1], S.pe2[1], r, Bo, O.store);
-                cpml_slot<NS, RS, R, P::exact>(z3, B, n, 3, si, false, y, x0, S.pb[1], S.pe[1], r, Bo, O.store);
-            }
-        }
-        si = slab_index(S, 2, x0, y, z);
-        if (si >= 0) {
-            void* B = O.psi_in[2];
-            void* Bo = O.psi_out ? O.psi_out[2] : nullptr;
-            const long long n = S.slab_cells[2];
-            cpml_slot<NS, RS, R, P::exact>(x3, B, n, 0, si, false, z, x0, S.pb[2], S.pe[2], r, Bo, O.store);
-            cpml_slot<NS, RS, R, P::exact>(z1, B, n, 1, si, false, z, x0, S.pb2[2], S.pe2[2], r, Bo, O.store);
-            cpml_slot<NS, RS, R, P::exact>(s3, B, n, 2, si, false, z, x0, S.pb2[2], S.pe2[2], r, Bo, O.store);
-            if constexpr (DIM == 3) cpml_slot<NS, RS, R, P::exact>(y3, B, n, 3, si, false, z, x0, S.pb[2], S.pe[2], r, Bo, O.store);
+            R (*const dx[NS])[4] = {&x1, &s1, &z2, &y2};
+            R (*const dy[NS])[4] = {&x2, &y1, &s2, &z3};
+            R (*const dz[NS])[4] = {&x3, &z1, &s3, &y3};
+            axis(dx, 0x3u, 0, x0);
+            axis(dy, 0x6u, 1, y);
+            axis(dz, 0x6u, 2, z);
+        } else {
+            R (*const dx[NS])[4] = {&x1, &s1, &z2};
+            R (*const dz[NS])[4] = {&x3, &z1, &s3};
+            axis(dx, 0x3u, 0, x0);
+            axis(dz, 0x6u, 2, z);
         }
     }
 
@@ -419,23 +457,56 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
 #pragma unroll
         for (int j = 0; j < 4; j++) { vw[j] = nw[j]; vu[j] = nu[j]; }
     };
-    if constexpr (!PRE) {
+    // FP32 loads every axis' coefficients and old velocities before the first
+    // axis' stores, so the chunk waits for them once.  Measured on B200 (us per
+    // step): 424 x 424 x 328 per-cell medium 3066 -> 2887, 296 x 296 x 232 1495 ->
+    // 1436, 4040 x 2040 per-cell 205.8 -> 202.9, indexed 162.6 -> 163.4.  The
+    // 3-byte and FP64 forms spill and lose: COMP16 2D 259 -> 321, CBF16 296 x
+    // 296 x 232 1681 -> 1791, FP64 168^3 814 -> 899.
+    constexpr bool kAhead = P::store == BP_PREC_FP32;
+    auto load_x = [&] {
         if (!med) P::template ld4<NC>(S.vc[VC_RHOF], S.vclo[VC_RHOF], c, rf);   // indexed: with the x group
-        load_axis(BP_F_VUX, BP_F_VWX, VC_RHO_X, VC_CC1_X, VC_CC2_X, rho_x, c1_x, c2_x, vu_x, vw_x);
+        load_axis(VC_RHO_X, VC_CC1_X, VC_CC2_X, rho_x, c1_x, c2_x);
+        src.template own<BP_F_VUX>(vu_x);
+        src.template own<BP_F_VWX>(vw_x);
+    };
+    auto load_y = [&] {
+        if constexpr (DIM == 3) {
+            load_axis(VC_RHO_Y, VC_CC1_Y, VC_CC2_Y, rho_y, c1_y, c2_y);
+            src.template own<BP_F_VUY>(vu_y);
+            src.template own<BP_F_VWY>(vw_y);
+        }
+    };
+    auto load_z = [&] {
+        load_axis(VC_RHO_Z, VC_CC1_Z, VC_CC2_Z, rho_z, c1_z, c2_z);
+        src.template own<BP_F_VUZ>(vu_z);
+        src.template own<BP_F_VWZ>(vw_z);
+    };
+    if constexpr (!PRE) {
+        load_x();
+        if constexpr (kAhead) {
+            if constexpr (DIM == 3) load_y();
+            load_z();
+        }
     }
     axis_update(sumx, s1, BP_F_VUX, BP_F_VWX, rho_x, c1_x, c2_x, vu_x, vw_x);
     if constexpr (DIM == 3) {
-        if constexpr (!PRE) load_axis(BP_F_VUY, BP_F_VWY, VC_RHO_Y, VC_CC1_Y, VC_CC2_Y, rho_y, c1_y, c2_y, vu_y, vw_y);
+        if constexpr (!PRE && !kAhead) load_y();
         axis_update(sumy, s2, BP_F_VUY, BP_F_VWY, rho_y, c1_y, c2_y, vu_y, vw_y);
     }
-    if constexpr (!PRE) load_axis(BP_F_VUZ, BP_F_VWZ, VC_RHO_Z, VC_CC1_Z, VC_CC2_Z, rho_z, c1_z, c2_z, vu_z, vw_z);
+    if constexpr (!PRE && !kAhead) load_z();
     axis_update(sumz, s3, BP_F_VUZ, BP_F_VWZ, rho_z, c1_z, c2_z, vu_z, vw_z);
 }
 
 template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
 __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
                                        unsigned mask, VState<typename P::real>& V) {
-    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, TailOut::v_of(S));
+    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, TailOut::v_of(S), ArraySrc<P>{S, c});
+}
+template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
+__device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
+                                       unsigned mask, VState<typename P::real>& V, const TailOut& O) {
+    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, O, ArraySrc<P>{S, c});
 }
 
 // ---------------------------------------------------------------------------
@@ -453,9 +524,9 @@ struct TState {
 };
 
 // On return T's old-stress members (op, oxx, ...) hold the new values.
-template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
+template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath, class Src>
 __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
-                                       unsigned mask, TState<typename P::real>& T, const TailOut& O) {
+                                       unsigned mask, TState<typename P::real>& T, const TailOut& O, const Src& src) {
     using R = typename P::real;
     auto &uxx = T.uxx, &uzz = T.uzz, &wx = T.wx, &wz = T.wz, &uxz = T.uxz, &uzx = T.uzx;
     auto &uyy = T.uyy, &wy = T.wy, &uxy = T.uxy, &uyx = T.uyx, &uyz = T.uyz, &uzy = T.uzy;
@@ -484,14 +555,14 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
                 P::template ld4<NC>(S.tc[TC_MUYZ], S.tclo[TC_MUYZ], c, myz);
             }
         }
-        P::ld4(S.f[BP_F_P], S.flo[BP_F_P], c, op);
-        P::ld4(S.f[BP_F_TXX], S.flo[BP_F_TXX], c, oxx);
-        P::ld4(S.f[BP_F_TZZ], S.flo[BP_F_TZZ], c, ozz);
-        P::ld4(S.f[BP_F_TXZ], S.flo[BP_F_TXZ], c, oxz);
+        src.template own<BP_F_P>(op);
+        src.template own<BP_F_TXX>(oxx);
+        src.template own<BP_F_TZZ>(ozz);
+        src.template own<BP_F_TXZ>(oxz);
         if constexpr (DIM == 3) {
-            P::ld4(S.f[BP_F_TYY], S.flo[BP_F_TYY], c, oyy);
-            P::ld4(S.f[BP_F_TXY], S.flo[BP_F_TXY], c, oxy);
-            P::ld4(S.f[BP_F_TYZ], S.flo[BP_F_TYZ], c, oyz);
+            src.template own<BP_F_TYY>(oyy);
+            src.template own<BP_F_TXY>(oxy);
+            src.template own<BP_F_TYZ>(oyz);
         }
         if constexpr (P::prec == BP_PREC_COMP16 && RS) {     // old state takes this step's rescale
             scale4(op, r); scale4(oxx, r); scale4(ozz, r); scale4(oxz, r);
@@ -509,34 +580,24 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
     // stored ψ/prev of this phase are old state and take the rescale r ----
     {
         constexpr int NS = DIM == 3 ? 4 : 3;
-        cidx si = slab_index(S, 0, x0, y, z);
-        if (si >= 0) {
-            void* B = O.psi_in[0];
-            const long long n = S.slab_cells[0];
-            cpml_slot<NS, RS, R, P::exact>(uxx, B, n, 0, si, true, x0, x0, S.pb[0], S.pe[0], r, nullptr, O.store);
-            cpml_slot<NS, RS, R, P::exact>(wx, B, n, 1, si, true, x0, x0, S.pb[0], S.pe[0], r, nullptr, O.store);
-            cpml_slot<NS, RS, R, P::exact>(uzx, B, n, 2, si, true, x0, x0, S.pb2[0], S.pe2[0], r, nullptr, O.store);
-            if constexpr (DIM == 3) cpml_slot<NS, RS, R, P::exact>(uyx, B, n, 3, si, true, x0, x0, S.pb2[0], S.pe2[0], r, nullptr, O.store);
-        }
+        auto axis = [&](R (*const (&d)[NS])[4], unsigned half, int a, int pos) {
+            const cidx si = slab_index(S, a, x0, y, z);
+            if (si >= 0)
+                cpml_axis<NS, RS, R, P::exact>(d, half, O.psi_in[a], S.slab_cells[a], si, a == 0, pos, x0, S.pb[a],
+                                               S.pe[a], S.pb2[a], S.pe2[a], r, nullptr, O.store);
+        };
         if constexpr (DIM == 3) {
-            si = slab_index(S, 1, x0, y, z);
-            if (si >= 0) {
-                void* B = O.psi_in[1];
-                const long long n = S.slab_cells[1];
-                cpml_slot<NS, RS, R, P::exact>(uyy, B, n, 0, si, false, y, x0, S.pb[1], S.pe[1], r, nullptr, O.store);
-                cpml_slot<NS, RS, R, P::exact>(wy, B, n, 1, si, false, y, x0, S.pb[1], S.pe[1], r, nullptr, O.store);
-                cpml_slot<NS, RS, R, P::exact>(uxy, B, n, 2, si, false, y, x0, S.pb2[1], S.pe2[1], r, nullptr, O.store);
-                cpml_slot<NS, RS, R, P::exact>(uzy, B, n, 3, si, false, y, x0, S.pb2[1], S.pe2[1], r, nullptr, O.store);
-            }
-        }
-        si = slab_index(S, 2, x0, y, z);
-        if (si >= 0) {
-            void* B = O.psi_in[2];
-            const long long n = S.slab_cells[2];
-            cpml_slot<NS, RS, R, P::exact>(uzz, B, n, 0, si, false, z, x0, S.pb[2], S.pe[2], r, nullptr, O.store);
-            cpml_slot<NS, RS, R, P::exact>(wz, B, n, 1, si, false, z, x0, S.pb[2], S.pe[2], r, nullptr, O.store);
-            cpml_slot<NS, RS, R, P::exact>(uxz, B, n, 2, si, false, z, x0, S.pb2[2], S.pe2[2], r, nullptr, O.store);
-            if constexpr (DIM == 3) cpml_slot<NS, RS, R, P::exact>(uyz, B, n, 3, si, false, z, x0, S.pb2[2], S.pe2[2], r, nullptr, O.store);
+            R (*const dx[NS])[4] = {&uxx, &wx, &uzx, &uyx};
+            R (*const dy[NS])[4] = {&uyy, &wy, &uxy, &uzy};
+            R (*const dz[NS])[4] = {&uzz, &wz, &uxz, &uyz};
+            axis(dx, 0xcu, 0, x0);
+            axis(dy, 0xcu, 1, y);
+            axis(dz, 0xcu, 2, z);
+        } else {
+            R (*const dx[NS])[4] = {&uxx, &wx, &uzx};
+            R (*const dz[NS])[4] = {&uzz, &wz, &uxz};
+            axis(dx, 0x4u, 0, x0);
+            axis(dz, 0x4u, 2, z);
         }
     }
 
@@ -640,7 +701,12 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
 __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
                                        unsigned mask, TState<typename P::real>& T) {
-    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, TailOut::t_of(S));
+    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, TailOut::t_of(S), ArraySrc<P>{S, c});
+}
+template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
+__device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
+                                       unsigned mask, TState<typename P::real>& T, const TailOut& O) {
+    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, O, ArraySrc<P>{S, c});
 }
 
 }  // namespace bpk

@@ -55,24 +55,21 @@ __device__ __forceinline__ int locate_shot(const ShotDesc* shots, int nshots, lo
 #ifndef BP_MINB_F64
 #define BP_MINB_F64 2
 #endif
-// 3D: uncapped, the kernels take 128-169 registers (1-2 CTAs per SM); capped
-// at 3 CTAs (80 registers, ~130 bytes spilled) the 192^3 order-2 and 200^3
-// order-4 FP32 steps run 1.75-2.1x faster on B200.  COMP16, taken one output
-// group at a time (v_chunk_g/t_chunk_g, next to no spills), is fastest at 4 CTAs
-// (64 registers) on the 552 x 552 x 424 and 200^3 grids; FP64 at 2 (128
-// registers; uncapped it takes 196-240, one CTA per SM).
+// 3D: uncapped, the kernels take 128-240 registers.  FP32 is fastest at 2 CTAs
+// (128 registers, no spills) now that a chunk's memory variables and
+// coefficients are loaded in batches: us per step on B200 at 3 -> 2 CTAs, 200^3
+// order 2 557 -> 417, order 4 588 -> 444, 104^3 order 4 123 -> 83, 140 x 130 x
+// 120 199 -> 147.  With the reference's rounding, whose divisions keep it busy
+// issuing, order 2 is fastest at 3 (192^3: 624 against 649 at 2), order 4 at 2
+// (200 x 190 x 180 per-cell medium: 747 -> 699).  COMP16, taken one output group
+// at a time (v_chunk_g/t_chunk_g, next to no spills), is fastest at 4 CTAs (64
+// registers) on the 552 x 552 x 424 and 200^3 grids; FP64 at 2 (128 registers;
+// uncapped it takes 196-240, one CTA per SM).
 #ifndef BP_MINB3_F32
-#define BP_MINB3_F32 3
+#define BP_MINB3_F32 2
 #endif
-// 3D FP32 on large grids (PolF32W, from kWideCells updated cells of a launch):
-// 2 CTAs (128 registers, no spills) for the T phase and the order-2 V phase,
-// measured on B200: the 552 x 552 x 424 order-2 step 5 % faster (16,716 ->
-// 17,507 Mcell-updates/s) and the uniform 300^3 order-2 T phase 15 % faster,
-// while the 192^3 order-2 reference run (7 M cells) is 13 % slower (26 % with
-// reference rounding) and keeps 3; the order-4 V phase keeps 3 everywhere
-// (12 % slower at 2)
-#ifndef BP_MINB3_F32_WIDE
-#define BP_MINB3_F32_WIDE 2
+#ifndef BP_MINB3_F32R
+#define BP_MINB3_F32R 3
 #endif
 #ifndef BP_MINB3_C16
 #define BP_MINB3_C16 4
@@ -94,7 +91,7 @@ __device__ __forceinline__ int locate_shot(const ShotDesc* shots, int nshots, lo
 template <int DIM, int ORD, class P, bool VPHASE>
 __host__ __device__ constexpr int phase_min_blocks() {
     if (P::store == BP_PREC_CBF16) return DIM == 3 ? BP_MINB3_B24 : (VPHASE ? BP_MINB_B24_V : BP_MINB_B24);
-    if (DIM == 3 && P::prec == BP_PREC_FP32 && P::wide) return (VPHASE && ORD == 4) ? BP_MINB3_F32 : BP_MINB3_F32_WIDE;
+    if (DIM == 3 && P::exact && ORD == 2) return BP_MINB3_F32R;
     if (DIM == 3) return P::prec == BP_PREC_FP32 ? BP_MINB3_F32 : P::prec == BP_PREC_COMP16 ? BP_MINB3_C16 : BP_MINB3_F64;
     return P::prec == BP_PREC_FP32 ? BP_MINB_F32
                                    : P::prec == BP_PREC_COMP16 ? (VPHASE ? BP_MINB_C16_V : BP_MINB_C16) : BP_MINB_F64;
@@ -129,175 +126,106 @@ __host__ __device__ constexpr bool read_only_loads() {
 }
 
 // ---------------------------------------------------------------------------
-// V phase for one 4-cell chunk: FD_V (Float/main.cu:103-191).
-// NCOK = false: no read-only-path loads (the interleaved step kernel reads
-// arrays that the same launch writes)
-template <int DIM, int ORD, class P, bool RS, bool NCOK = true>
-__device__ __forceinline__ void v_chunk(const ShotDesc& S, int x0, int y, int z, typename P::real r,
-                                        unsigned mask) {
+// Where a chunk's field values come from.  GlobalSrc loads them from the field
+// arrays (NC: through the read-only path); AsyncSrc (async.cuh) from the
+// warp's shared-memory slots, which asynchronous copies have filled.
+// span: cells x0 - HW .. x0 + 3 + HW of the chunk's row; rows: the chunk's cells
+// in rows -HW .. HW along y (AX 1) or z (AX 2); own: the chunk's cells.
+template <int ORD, class P, bool NC>
+struct GlobalSrc {
     using R = typename P::real;
-    const cidx sy = S.pitch, sz = S.plane;
-    const cidx c = x0 + y * sy + z * sz;
-    const cidx row = c - x0;
-
-    VState<R> V;
-    // an indexed medium's tuple indices first: their load overlaps the field loads
-    if (med_on<P>(S)) V.mids = med_ids(S, c);
-    auto &x1 = V.x1, &x3 = V.x3, &s1 = V.s1, &z1 = V.z1, &z2 = V.z2, &s3 = V.s3;
-    auto &x2 = V.x2, &y1 = V.y1, &y2 = V.y2, &y3 = V.y3, &s2 = V.s2, &z3 = V.z3;
-
-    // ---- derivatives of the old stresses (x1..s3, Float/main.cu:115-128) ----
-    {
-        R v[4 + ORD];
-        load_span<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TXX], S.flo[BP_F_TXX], row, x0, S.nx, v);       // txx: D+x
-#pragma unroll
-        for (int j = 0; j < 4; j++) x1[j] = deriv_div<P>(dfwd<ORD>(v, j), S);
-        load_span<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_P], S.flo[BP_F_P], row, x0, S.nx, v);           // p: D+x
-#pragma unroll
-        for (int j = 0; j < 4; j++) s1[j] = deriv_div<P>(dfwd<ORD>(v, j), S);
-        load_span<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TXZ], S.flo[BP_F_TXZ], row, x0, S.nx, v);       // txz: D-x
-#pragma unroll
-        for (int j = 0; j < 4; j++) z2[j] = deriv_div<P>(dbwd<ORD>(v, j), S);
-        R a[ORD + 1][4];
-        load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TXZ], S.flo[BP_F_TXZ], c, sz, a);               // txz: D-z
-#pragma unroll
-        for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-            for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-            x3[j] = deriv_z<P, false>(rbwd<ORD>(t), S, z); }
-        load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TZZ], S.flo[BP_F_TZZ], c, sz, a);               // tzz: D+z
-#pragma unroll
-        for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-            for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-            z1[j] = deriv_z<P, true>(rfwd<ORD>(t), S, z); }
-        load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_P], S.flo[BP_F_P], c, sz, a);                   // p: D+z
-#pragma unroll
-        for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-            for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-            s3[j] = deriv_z<P, true>(rfwd<ORD>(t), S, z); }
-        if constexpr (DIM == 3) {
-            load_span<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TXY], S.flo[BP_F_TXY], row, x0, S.nx, v);   // txy: D-x
-#pragma unroll
-            for (int j = 0; j < 4; j++) y2[j] = deriv_div<P>(dbwd<ORD>(v, j), S);
-            load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TXY], S.flo[BP_F_TXY], c, sy, a);           // txy: D-y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                x2[j] = deriv_div<P>(rbwd<ORD>(t), S); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TYY], S.flo[BP_F_TYY], c, sy, a);           // tyy: D+y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                y1[j] = deriv_div<P>(rfwd<ORD>(t), S); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TYZ], S.flo[BP_F_TYZ], c, sz, a);           // tyz: D-z
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                y3[j] = deriv_z<P, false>(rbwd<ORD>(t), S, z); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_TYZ], S.flo[BP_F_TYZ], c, sy, a);           // tyz: D-y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                z3[j] = deriv_div<P>(rbwd<ORD>(t), S); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, true>() && NCOK)>(S.f[BP_F_P], S.flo[BP_F_P], c, sy, a);               // p: D+y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                s2[j] = deriv_div<P>(rfwd<ORD>(t), S); }
-        }
+    const ShotDesc& S;
+    cidx c;
+    int x0;
+    template <int F>
+    __device__ __forceinline__ void span(R (&v)[4 + ORD]) const {
+        load_span<ORD, P, NC>(S.f[F], S.flo[F], c - x0, x0, S.nx, v);
     }
-    v_tail<DIM, ORD, P, false, RS, (read_only_loads<DIM, P, true>() && NCOK)>(S, c, x0, y, z, r, mask, V);
+    template <int F, int AX>
+    __device__ __forceinline__ void rows(R (&a)[ORD + 1][4]) const {
+        load_rows<ORD, P, NC>(S.f[F], S.flo[F], c, AX == 1 ? S.pitch : (cidx)S.plane, a);
+    }
+    template <int F>
+    __device__ __forceinline__ void own(R (&v)[4]) const {
+        P::ld4(S.f[F], S.flo[F], c, v);
+    }
+};
+
+// Difference along x of field F at the chunk (FWD: at x + 1/2), divided by H.
+template <int ORD, class P, int F, bool FWD, class Src>
+__device__ __forceinline__ void d_span(const ShotDesc& S, const Src& src, typename P::real (&d)[4]) {
+    typename P::real v[4 + ORD];
+    src.template span<F>(v);
+#pragma unroll
+    for (int j = 0; j < 4; j++) d[j] = deriv_div<P>(FWD ? dfwd<ORD>(v, j) : dbwd<ORD>(v, j), S);
+}
+// Difference across rows (AX 1: y, 2: z) of field F at the chunk, divided by
+// the spacing.
+template <int ORD, class P, int F, int AX, bool FWD, class Src>
+__device__ __forceinline__ void d_rows(const ShotDesc& S, const Src& src, int z, typename P::real (&d)[4]) {
+    using R = typename P::real;
+    R a[ORD + 1][4];
+    src.template rows<F, AX>(a);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        R t[ORD + 1];
+#pragma unroll
+        for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
+        const R q = FWD ? rfwd<ORD>(t) : rbwd<ORD>(t);
+        if constexpr (AX == 2) d[j] = deriv_z<P, FWD>(q, S, z);
+        else d[j] = deriv_div<P>(q, S);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// V phase for one 4-cell chunk: FD_V (Float/main.cu:103-191).
+// NC: read-only-path loads of the coefficients; ids: the chunk's tuple indices
+// (indexed medium)
+template <int DIM, int ORD, class P, bool RS, bool NC, class Src>
+__device__ __forceinline__ void v_chunk(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                        typename P::real r, unsigned mask, unsigned ids) {
+    VState<typename P::real> V;
+    V.mids = ids;
+    // ---- derivatives of the old stresses (x1..s3, Float/main.cu:115-128) ----
+    d_span<ORD, P, BP_F_TXX, true>(S, src, V.x1);
+    d_span<ORD, P, BP_F_P, true>(S, src, V.s1);
+    d_span<ORD, P, BP_F_TXZ, false>(S, src, V.z2);
+    d_rows<ORD, P, BP_F_TXZ, 2, false>(S, src, z, V.x3);
+    d_rows<ORD, P, BP_F_TZZ, 2, true>(S, src, z, V.z1);
+    d_rows<ORD, P, BP_F_P, 2, true>(S, src, z, V.s3);
+    if constexpr (DIM == 3) {
+        d_span<ORD, P, BP_F_TXY, false>(S, src, V.y2);
+        d_rows<ORD, P, BP_F_TXY, 1, false>(S, src, z, V.x2);
+        d_rows<ORD, P, BP_F_TYY, 1, true>(S, src, z, V.y1);
+        d_rows<ORD, P, BP_F_TYZ, 2, false>(S, src, z, V.y3);
+        d_rows<ORD, P, BP_F_TYZ, 1, false>(S, src, z, V.z3);
+        d_rows<ORD, P, BP_F_P, 1, true>(S, src, z, V.s2);
+    }
+    v_tail<DIM, ORD, P, false, RS, NC>(S, c, x0, y, z, r, mask, V, TailOut::v_of(S), src);
 }
 
 // ---------------------------------------------------------------------------
 // T phase for one 4-cell chunk: FD_T (Float/main.cu:232-294).
-template <int DIM, int ORD, class P, bool RS, bool NCOK = true>
-__device__ __forceinline__ void t_chunk(const ShotDesc& S, int x0, int y, int z, typename P::real r,
-                                        unsigned mask) {
-    using R = typename P::real;
-    const cidx sy = S.pitch, sz = S.plane;
-    const cidx c = x0 + y * sy + z * sz;
-    const cidx row = c - x0;
-
-    TState<R> T;
-    if (med_on<P>(S)) T.mids = med_ids(S, c);
-    auto &uxx = T.uxx, &uzz = T.uzz, &wx = T.wx, &wz = T.wz, &uxz = T.uxz, &uzx = T.uzx;
-    auto &uyy = T.uyy, &wy = T.wy, &uxy = T.uxy, &uyx = T.uyx, &uyz = T.uyz, &uzy = T.uzy;
-
-    {
-        R v[4 + ORD];
-        R a[ORD + 1][4];
-        load_span<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUX], S.flo[BP_F_VUX], row, x0, S.nx, v);       // vux: D-x
-#pragma unroll
-        for (int j = 0; j < 4; j++) uxx[j] = deriv_div<P>(dbwd<ORD>(v, j), S);
-        load_span<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VWX], S.flo[BP_F_VWX], row, x0, S.nx, v);       // vwx: D-x
-#pragma unroll
-        for (int j = 0; j < 4; j++) wx[j] = deriv_div<P>(dbwd<ORD>(v, j), S);
-        load_span<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUZ], S.flo[BP_F_VUZ], row, x0, S.nx, v);       // vuz: D+x
-#pragma unroll
-        for (int j = 0; j < 4; j++) uzx[j] = deriv_div<P>(dfwd<ORD>(v, j), S);
-        load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUZ], S.flo[BP_F_VUZ], c, sz, a);               // vuz: D-z
-#pragma unroll
-        for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-            for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-            uzz[j] = deriv_z<P, false>(rbwd<ORD>(t), S, z); }
-        load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VWZ], S.flo[BP_F_VWZ], c, sz, a);               // vwz: D-z
-#pragma unroll
-        for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-            for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-            wz[j] = deriv_z<P, false>(rbwd<ORD>(t), S, z); }
-        load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUX], S.flo[BP_F_VUX], c, sz, a);               // vux: D+z
-#pragma unroll
-        for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-            for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-            uxz[j] = deriv_z<P, true>(rfwd<ORD>(t), S, z); }
-        if constexpr (DIM == 3) {
-            load_span<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUY], S.flo[BP_F_VUY], row, x0, S.nx, v);   // vuy: D+x
-#pragma unroll
-            for (int j = 0; j < 4; j++) uyx[j] = deriv_div<P>(dfwd<ORD>(v, j), S);
-            load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUY], S.flo[BP_F_VUY], c, sy, a);           // vuy: D-y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                uyy[j] = deriv_div<P>(rbwd<ORD>(t), S); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VWY], S.flo[BP_F_VWY], c, sy, a);           // vwy: D-y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                wy[j] = deriv_div<P>(rbwd<ORD>(t), S); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUX], S.flo[BP_F_VUX], c, sy, a);           // vux: D+y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                uxy[j] = deriv_div<P>(rfwd<ORD>(t), S); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUY], S.flo[BP_F_VUY], c, sz, a);           // vuy: D+z
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                uyz[j] = deriv_z<P, true>(rfwd<ORD>(t), S, z); }
-            load_rows<ORD, P, (read_only_loads<DIM, P, false>() && NCOK)>(S.f[BP_F_VUZ], S.flo[BP_F_VUZ], c, sy, a);           // vuz: D+y
-#pragma unroll
-            for (int j = 0; j < 4; j++) { R t[ORD + 1];
-#pragma unroll
-                for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-                uzy[j] = deriv_div<P>(rfwd<ORD>(t), S); }
-        }
+template <int DIM, int ORD, class P, bool RS, bool NC, class Src>
+__device__ __forceinline__ void t_chunk(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                        typename P::real r, unsigned mask, unsigned ids) {
+    TState<typename P::real> T;
+    T.mids = ids;
+    d_span<ORD, P, BP_F_VUX, false>(S, src, T.uxx);
+    d_span<ORD, P, BP_F_VWX, false>(S, src, T.wx);
+    d_span<ORD, P, BP_F_VUZ, true>(S, src, T.uzx);
+    d_rows<ORD, P, BP_F_VUZ, 2, false>(S, src, z, T.uzz);
+    d_rows<ORD, P, BP_F_VWZ, 2, false>(S, src, z, T.wz);
+    d_rows<ORD, P, BP_F_VUX, 2, true>(S, src, z, T.uxz);
+    if constexpr (DIM == 3) {
+        d_span<ORD, P, BP_F_VUY, true>(S, src, T.uyx);
+        d_rows<ORD, P, BP_F_VUY, 1, false>(S, src, z, T.uyy);
+        d_rows<ORD, P, BP_F_VWY, 1, false>(S, src, z, T.wy);
+        d_rows<ORD, P, BP_F_VUX, 1, true>(S, src, z, T.uxy);
+        d_rows<ORD, P, BP_F_VUY, 2, true>(S, src, z, T.uyz);
+        d_rows<ORD, P, BP_F_VUZ, 1, true>(S, src, z, T.uzy);
     }
-    t_tail<DIM, ORD, P, false, RS, (read_only_loads<DIM, P, false>() && NCOK)>(S, c, x0, y, z, r, mask, T);
+    t_tail<DIM, ORD, P, false, RS, NC>(S, c, x0, y, z, r, mask, T, TailOut::t_of(S), src);
 }
 
 // ---------------------------------------------------------------------------
@@ -340,31 +268,6 @@ __host__ __device__ constexpr bool grouped() {
     return (m >> (VPHASE ? 0 : 1)) & 1;
 }
 
-// Difference along x of one field at the chunk (span load), divided by H.
-template <int ORD, class P, bool FWD>
-__device__ __forceinline__ void d_span(const ShotDesc& S, int f, cidx row, int x0,
-                                       typename P::real (&d)[4]) {
-    typename P::real v[4 + ORD];
-    load_span<ORD, P>(S.f[f], S.flo[f], row, x0, S.nx, v);
-#pragma unroll
-    for (int j = 0; j < 4; j++) d[j] = deriv_div<P>(FWD ? dfwd<ORD>(v, j) : dbwd<ORD>(v, j), S);
-}
-// Difference across rows (y or z) of one field at the chunk, divided by H.
-template <int ORD, class P, bool FWD>
-__device__ __forceinline__ void d_rows(const ShotDesc& S, int f, cidx c, cidx stride,
-                                       typename P::real (&d)[4]) {
-    static_assert(!P::graded, "the grouped forms take a uniform grid (FP32 runs the whole-chunk form)");
-    using R = typename P::real;
-    R a[ORD + 1][4];
-    load_rows<ORD, P>(S.f[f], S.flo[f], c, stride, a);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        R t[ORD + 1];
-#pragma unroll
-        for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
-        d[j] = deriv_div<P>(FWD ? rfwd<ORD>(t) : rbwd<ORD>(t), S);
-    }
-}
 // Masked cells feed zero derivatives into the memory variables.
 template <class R>
 __device__ __forceinline__ void mask0(R (&d)[4], unsigned mask) {
@@ -386,29 +289,29 @@ __device__ __forceinline__ void cpml_g(const ShotDesc& S, void* const (&psi)[3],
 
 // One velocity component AX (0 = x, 1 = y, 2 = z) of the V phase
 // (Float/main.cu:103-191 for that component).
-template <int DIM, int ORD, class P, bool RS, int AX>
-__device__ __forceinline__ void v_comp(const ShotDesc& S, cidx c, cidx row, int x0, int y, int z,
-                                       typename P::real r, unsigned mask, const typename P::real (&rf)[4]) {
+template <int DIM, int ORD, class P, bool RS, int AX, class Src>
+__device__ __forceinline__ void v_comp(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                       typename P::real r, unsigned mask, unsigned ids,
+                                       const typename P::real (&rf)[4]) {
     using R = typename P::real;
-    const cidx sy = S.pitch, sz = S.plane;
     // dx, dy, dz: the stress derivatives summed into this component (dy in 3D
     // only); dp: the pressure derivative along AX.  Slots as in v_tail.
     R dx[4], dy[4], dz[4], dp[4];
     if constexpr (AX == 0) {
-        d_span<ORD, P, true>(S, BP_F_TXX, row, x0, dx);                          // x1
-        if constexpr (DIM == 3) d_rows<ORD, P, false>(S, BP_F_TXY, c, sy, dy);   // x2
-        d_rows<ORD, P, false>(S, BP_F_TXZ, c, sz, dz);                           // x3
-        d_span<ORD, P, true>(S, BP_F_P, row, x0, dp);                            // s1
+        d_span<ORD, P, BP_F_TXX, true>(S, src, dx);                          // x1
+        if constexpr (DIM == 3) d_rows<ORD, P, BP_F_TXY, 1, false>(S, src, z, dy);   // x2
+        d_rows<ORD, P, BP_F_TXZ, 2, false>(S, src, z, dz);                           // x3
+        d_span<ORD, P, BP_F_P, true>(S, src, dp);                            // s1
     } else if constexpr (AX == 1) {
-        d_span<ORD, P, false>(S, BP_F_TXY, row, x0, dx);                         // y2
-        d_rows<ORD, P, true>(S, BP_F_TYY, c, sy, dy);                            // y1
-        d_rows<ORD, P, false>(S, BP_F_TYZ, c, sz, dz);                           // y3
-        d_rows<ORD, P, true>(S, BP_F_P, c, sy, dp);                              // s2
+        d_span<ORD, P, BP_F_TXY, false>(S, src, dx);                         // y2
+        d_rows<ORD, P, BP_F_TYY, 1, true>(S, src, z, dy);                            // y1
+        d_rows<ORD, P, BP_F_TYZ, 2, false>(S, src, z, dz);                           // y3
+        d_rows<ORD, P, BP_F_P, 1, true>(S, src, z, dp);                              // s2
     } else {
-        d_span<ORD, P, false>(S, BP_F_TXZ, row, x0, dx);                         // z2
-        if constexpr (DIM == 3) d_rows<ORD, P, false>(S, BP_F_TYZ, c, sy, dy);   // z3
-        d_rows<ORD, P, true>(S, BP_F_TZZ, c, sz, dz);                            // z1
-        d_rows<ORD, P, true>(S, BP_F_P, c, sz, dp);                              // s3
+        d_span<ORD, P, BP_F_TXZ, false>(S, src, dx);                         // z2
+        if constexpr (DIM == 3) d_rows<ORD, P, BP_F_TYZ, 1, false>(S, src, z, dy);   // z3
+        d_rows<ORD, P, BP_F_TZZ, 2, true>(S, src, z, dz);                            // z1
+        d_rows<ORD, P, BP_F_P, 2, true>(S, src, z, dp);                              // s3
     }
     if constexpr (P::prec == BP_PREC_COMP16 && RS) {
         scale4(dx, r); scale4(dz, r); scale4(dp, r);
@@ -450,11 +353,11 @@ __device__ __forceinline__ void v_comp(const ShotDesc& S, cidx c, cidx row, int 
     constexpr int cc1 = AX == 0 ? VC_CC1_X : AX == 1 ? VC_CC1_Y : VC_CC1_Z;
     constexpr int cc2 = AX == 0 ? VC_CC2_X : AX == 1 ? VC_CC2_Y : VC_CC2_Z;
     R rho[4], c1[4], c2[4], vu[4], vw[4], nu[4], nw[4];
-    vcoef4<P>(S, crho, c, rho);
-    vcoef4<P>(S, cc1, c, c1);
-    vcoef4<P>(S, cc2, c, c2);
-    P::ld4(S.f[fu], S.flo[fu], c, vu);
-    P::ld4(S.f[fw], S.flo[fw], c, vw);
+    vcoef4<P>(S, crho, c, ids, rho);
+    vcoef4<P>(S, cc1, c, ids, c1);
+    vcoef4<P>(S, cc2, c, ids, c2);
+    src.template own<fu>(vu);
+    src.template own<fw>(vw);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         if constexpr (P::prec == BP_PREC_COMP16) {
@@ -476,24 +379,20 @@ __device__ __forceinline__ void v_comp(const ShotDesc& S, cidx c, cidx row, int 
     P::st4(S.f[fu], S.flo[fu], c, nu);
 }
 
-template <int DIM, int ORD, class P, bool RS>
-__device__ __forceinline__ void v_chunk_g(const ShotDesc& S, int x0, int y, int z, typename P::real r,
-                                          unsigned mask) {
-    using R = typename P::real;
-    const cidx c = x0 + y * S.pitch + z * (cidx)S.plane;
-    const cidx row = c - x0;
-    R rf[4];
-    vcoef4<P>(S, VC_RHOF, c, rf);
-    v_comp<DIM, ORD, P, RS, 0>(S, c, row, x0, y, z, r, mask, rf);
-    if constexpr (DIM == 3) v_comp<DIM, ORD, P, RS, 1>(S, c, row, x0, y, z, r, mask, rf);
-    v_comp<DIM, ORD, P, RS, 2>(S, c, row, x0, y, z, r, mask, rf);
+template <int DIM, int ORD, class P, bool RS, class Src>
+__device__ __forceinline__ void v_chunk_g(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                          typename P::real r, unsigned mask, unsigned ids) {
+    typename P::real rf[4];
+    vcoef4<P>(S, VC_RHOF, c, ids, rf);
+    v_comp<DIM, ORD, P, RS, 0>(S, src, c, x0, y, z, r, mask, ids, rf);
+    if constexpr (DIM == 3) v_comp<DIM, ORD, P, RS, 1>(S, src, c, x0, y, z, r, mask, ids, rf);
+    v_comp<DIM, ORD, P, RS, 2>(S, src, c, x0, y, z, r, mask, ids, rf);
 }
 
 // Old value of a stress field at the chunk, with this step's rescale.
-template <class P, bool RS>
-__device__ __forceinline__ void ld_old(const ShotDesc& S, int f, cidx c, typename P::real r,
-                                       typename P::real (&o)[4]) {
-    P::ld4(S.f[f], S.flo[f], c, o);
+template <int F, class P, bool RS, class Src>
+__device__ __forceinline__ void ld_old(const Src& src, typename P::real r, typename P::real (&o)[4]) {
+    src.template own<F>(o);
     if constexpr (P::prec == BP_PREC_COMP16 && RS) scale4(o, r);
 }
 template <class P>
@@ -507,21 +406,20 @@ __device__ __forceinline__ void st_new(const ShotDesc& S, int f, cidx c, unsigne
 
 // One shear stress of the T phase: SH 0 = txy, 1 = tyz (3D only), 2 = txz
 // (Float/main.cu:232-294 for that stress).
-template <int DIM, int ORD, class P, bool RS, int SH>
-__device__ __forceinline__ void t_shear(const ShotDesc& S, cidx c, cidx row, int x0, int y, int z,
-                                        typename P::real r, unsigned mask, void* const (&psi)[3]) {
+template <int DIM, int ORD, class P, bool RS, int SH, class Src>
+__device__ __forceinline__ void t_shear(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                        typename P::real r, unsigned mask, unsigned ids, void* const (&psi)[3]) {
     using R = typename P::real;
-    const cidx sy = S.pitch, sz = S.plane;
     R a[4], b[4];    // the two derivatives, in the order of the update's sum
     if constexpr (SH == 0) {
-        d_rows<ORD, P, true>(S, BP_F_VUX, c, sy, a);        // uxy
-        d_span<ORD, P, true>(S, BP_F_VUY, row, x0, b);      // uyx
+        d_rows<ORD, P, BP_F_VUX, 1, true>(S, src, z, a);        // uxy
+        d_span<ORD, P, BP_F_VUY, true>(S, src, b);      // uyx
     } else if constexpr (SH == 1) {
-        d_rows<ORD, P, true>(S, BP_F_VUY, c, sz, a);        // uyz
-        d_rows<ORD, P, true>(S, BP_F_VUZ, c, sy, b);        // uzy
+        d_rows<ORD, P, BP_F_VUY, 2, true>(S, src, z, a);        // uyz
+        d_rows<ORD, P, BP_F_VUZ, 1, true>(S, src, z, b);        // uzy
     } else {
-        d_rows<ORD, P, true>(S, BP_F_VUX, c, sz, a);        // uxz
-        d_span<ORD, P, true>(S, BP_F_VUZ, row, x0, b);      // uzx
+        d_rows<ORD, P, BP_F_VUX, 2, true>(S, src, z, a);        // uxz
+        d_span<ORD, P, BP_F_VUZ, true>(S, src, b);      // uzx
     }
     mask0(a, mask); mask0(b, mask);
     if constexpr (SH == 0) {
@@ -537,8 +435,8 @@ __device__ __forceinline__ void t_shear(const ShotDesc& S, cidx c, cidx row, int
     constexpr int f = SH == 0 ? BP_F_TXY : SH == 1 ? BP_F_TYZ : BP_F_TXZ;
     constexpr int cm = SH == 0 ? TC_MUXY : SH == 1 ? TC_MUYZ : TC_MUXZ;
     R mu[4], o[4], n[4];
-    tcoef4<P>(S, cm, c, mu);
-    ld_old<P, RS>(S, f, c, r, o);
+    tcoef4<P>(S, cm, c, ids, mu);
+    ld_old<f, P, RS>(src, r, o);
     const R dt = S.dtr<R>();
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -548,30 +446,27 @@ __device__ __forceinline__ void t_shear(const ShotDesc& S, cidx c, cidx row, int
     st_new<P>(S, f, c, mask, n, o);
 }
 
-template <int DIM, int ORD, class P, bool RS>
-__device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int z, typename P::real r,
-                                          unsigned mask) {
+template <int DIM, int ORD, class P, bool RS, class Src>
+__device__ __forceinline__ void t_chunk_g(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                          typename P::real r, unsigned mask, unsigned ids) {
     using R = typename P::real;
-    const cidx sy = S.pitch, sz = S.plane;
-    const cidx c = x0 + y * sy + z * sz;
-    const cidx row = c - x0;
     void* const psi[3] = {S.psiT[0], S.psiT[1], S.psiT[2]};
     if constexpr (DIM == 3) {
-        t_shear<DIM, ORD, P, RS, 0>(S, c, row, x0, y, z, r, mask, psi);
-        t_shear<DIM, ORD, P, RS, 1>(S, c, row, x0, y, z, r, mask, psi);
+        t_shear<DIM, ORD, P, RS, 0>(S, src, c, x0, y, z, r, mask, ids, psi);
+        t_shear<DIM, ORD, P, RS, 1>(S, src, c, x0, y, z, r, mask, ids, psi);
     }
-    t_shear<DIM, ORD, P, RS, 2>(S, c, row, x0, y, z, r, mask, psi);
+    t_shear<DIM, ORD, P, RS, 2>(S, src, c, x0, y, z, r, mask, ids, psi);
 
     // normal stresses and pressure: the divergence derivatives (uyy, wy in 3D)
     R uxx[4], uyy[4], uzz[4], wx[4], wy[4], wz[4];
-    d_span<ORD, P, false>(S, BP_F_VUX, row, x0, uxx);
-    d_span<ORD, P, false>(S, BP_F_VWX, row, x0, wx);
+    d_span<ORD, P, BP_F_VUX, false>(S, src, uxx);
+    d_span<ORD, P, BP_F_VWX, false>(S, src, wx);
     if constexpr (DIM == 3) {
-        d_rows<ORD, P, false>(S, BP_F_VUY, c, sy, uyy);
-        d_rows<ORD, P, false>(S, BP_F_VWY, c, sy, wy);
+        d_rows<ORD, P, BP_F_VUY, 1, false>(S, src, z, uyy);
+        d_rows<ORD, P, BP_F_VWY, 1, false>(S, src, z, wy);
     }
-    d_rows<ORD, P, false>(S, BP_F_VUZ, c, sz, uzz);
-    d_rows<ORD, P, false>(S, BP_F_VWZ, c, sz, wz);
+    d_rows<ORD, P, BP_F_VUZ, 2, false>(S, src, z, uzz);
+    d_rows<ORD, P, BP_F_VWZ, 2, false>(S, src, z, wz);
     mask0(uxx, mask); mask0(wx, mask); mask0(uzz, mask); mask0(wz, mask);
     if constexpr (DIM == 3) { mask0(uyy, mask); mask0(wy, mask); }
     {
@@ -589,9 +484,9 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int 
     }
     R cC[4], cM[4], cH[4], cH2[4], o[4], n[4];
     const R dt = S.dtr<R>();
-    tcoef4<P>(S, TC_C, c, cC);
-    tcoef4<P>(S, TC_M, c, cM);
-    ld_old<P, RS>(S, BP_F_P, c, r, o);
+    tcoef4<P>(S, TC_C, c, ids, cC);
+    tcoef4<P>(S, TC_M, c, ids, cM);
+    ld_old<BP_F_P, P, RS>(src, r, o);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         if constexpr (DIM == 3) {
@@ -607,9 +502,9 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int 
         }
     }
     st_new<P>(S, BP_F_P, c, mask, n, o);
-    tcoef4<P>(S, TC_H, c, cH);
-    tcoef4<P>(S, TC_H2U, c, cH2);
-    ld_old<P, RS>(S, BP_F_TXX, c, r, o);
+    tcoef4<P>(S, TC_H, c, ids, cH);
+    tcoef4<P>(S, TC_H2U, c, ids, cH2);
+    ld_old<BP_F_TXX, P, RS>(src, r, o);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         if constexpr (DIM == 3) {
@@ -626,7 +521,7 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int 
     }
     st_new<P>(S, BP_F_TXX, c, mask, n, o);
     if constexpr (DIM == 3) {
-        ld_old<P, RS>(S, BP_F_TYY, c, r, o);
+        ld_old<BP_F_TYY, P, RS>(src, r, o);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
@@ -636,7 +531,7 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int 
         }
         st_new<P>(S, BP_F_TYY, c, mask, n, o);
     }
-    ld_old<P, RS>(S, BP_F_TZZ, c, r, o);
+    ld_old<BP_F_TZZ, P, RS>(src, r, o);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         if constexpr (DIM == 3) {
@@ -655,43 +550,71 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, int x0, int y, int 
 }
 
 // ---------------------------------------------------------------------------
-// One chunk of one phase: cells x0 .. x0 + 3 of row (y, z) (it: the step index,
-// r: the COMP16 rescale factor of that step), nothing if the phase updates none
-// of them.  post (T phase only): the chunk also records the receivers in its
-// cells and, if it holds the source cell, injects the next source sample, in
-// place of the post-step kernel k_post.
-template <int DIM, int ORD, class P, bool VPHASE, bool NCOK>
-__device__ __forceinline__ void chunk_unit(const ShotDesc& S, int x0, int y, int z, typename P::real r, int it,
-                                           int post) {
-    using R = typename P::real;
+// The cells of the chunk at x0 the phases update, as a 4-bit mask (0: none).
+template <int ORD>
+__device__ __forceinline__ unsigned chunk_mask(const ShotDesc& S, int x0) {
     const int hw = ORD / 2;
-    if (z < hw || z >= S.nz - hw) return;
-    if (DIM == 3 && (y < hw || y >= S.ny - hw)) return;
-    if (x0 >= S.nx - hw || x0 + 3 < hw) return;
     unsigned mask = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++)
         if (x0 + j >= hw && x0 + j < S.nx - hw) mask |= 1u << j;
+    return mask;
+}
+// Whether the phases update row (y, z).
+template <int DIM, int ORD>
+__device__ __forceinline__ bool row_updated(const ShotDesc& S, int y, int z) {
+    const int hw = ORD / 2;
+    return z >= hw && z < S.nz - hw && (DIM == 2 || (y >= hw && y < S.ny - hw));
+}
+
+// One chunk of one phase: cells x0 .. x0 + 3 of row (y, z), mask of them updated
+// (it: the step index, r: the COMP16 rescale factor of that step).  post (T
+// phase only): the chunk also records the receivers in its cells and, if it
+// holds the source cell, injects the next source sample, in place of the
+// post-step kernel k_post.
+template <int DIM, int ORD, class P, bool VPHASE, bool NC, bool GROUPED, class Src>
+__device__ __forceinline__ void chunk_work(const ShotDesc& S, const Src& src, cidx c, int x0, int y, int z,
+                                           typename P::real r, unsigned mask, unsigned ids, int it, int post) {
+    using R = typename P::real;
+    constexpr bool C16 = P::prec == BP_PREC_COMP16;
     // COMP16: the rescale products only on the steps whose factor is not
     // exactly 1 (a uniform branch; the products are never fused, so both
     // forms give the same bits when r == 1)
-    if constexpr (grouped<DIM, P, VPHASE>()) {
-        if (P::prec == BP_PREC_COMP16 && (r != (R)1 || !BP_RS_SPLIT)) {
-            if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, P::prec == BP_PREC_COMP16>(S, x0, y, z, r, mask);
-            else t_chunk_g<DIM, ORD, P, P::prec == BP_PREC_COMP16>(S, x0, y, z, r, mask);
+    if (C16 && (r != (R)1 || !BP_RS_SPLIT)) {
+        if constexpr (GROUPED) {
+            if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, C16>(S, src, c, x0, y, z, r, mask, ids);
+            else t_chunk_g<DIM, ORD, P, C16>(S, src, c, x0, y, z, r, mask, ids);
         } else {
-            if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, false>(S, x0, y, z, r, mask);
-            else t_chunk_g<DIM, ORD, P, false>(S, x0, y, z, r, mask);
+            if constexpr (VPHASE) v_chunk<DIM, ORD, P, C16, NC>(S, src, c, x0, y, z, r, mask, ids);
+            else t_chunk<DIM, ORD, P, C16, NC>(S, src, c, x0, y, z, r, mask, ids);
         }
-    } else if (P::prec == BP_PREC_COMP16 && (r != (R)1 || !BP_RS_SPLIT)) {
-        if constexpr (VPHASE) v_chunk<DIM, ORD, P, P::prec == BP_PREC_COMP16, NCOK>(S, x0, y, z, r, mask);
-        else t_chunk<DIM, ORD, P, P::prec == BP_PREC_COMP16, NCOK>(S, x0, y, z, r, mask);
     } else {
-        if constexpr (VPHASE) v_chunk<DIM, ORD, P, false, NCOK>(S, x0, y, z, r, mask);
-        else t_chunk<DIM, ORD, P, false, NCOK>(S, x0, y, z, r, mask);
+        if constexpr (GROUPED) {
+            if constexpr (VPHASE) v_chunk_g<DIM, ORD, P, false>(S, src, c, x0, y, z, r, mask, ids);
+            else t_chunk_g<DIM, ORD, P, false>(S, src, c, x0, y, z, r, mask, ids);
+        } else {
+            if constexpr (VPHASE) v_chunk<DIM, ORD, P, false, NC>(S, src, c, x0, y, z, r, mask, ids);
+            else t_chunk<DIM, ORD, P, false, NC>(S, src, c, x0, y, z, r, mask, ids);
+        }
     }
     if constexpr (!VPHASE)
-        if (post) post_chunk<DIM, P>(S, it, x0 + y * (cidx)S.pitch + z * (cidx)S.plane, x0, y, z);
+        if (post) post_chunk<DIM, P>(S, it, c, x0, y, z);
+}
+// The same from the field arrays.  NCOK = false: no read-only-path loads (the
+// interleaved step kernel reads arrays that the same launch writes).
+template <int DIM, int ORD, class P, bool VPHASE, bool NCOK>
+__device__ __forceinline__ void chunk_unit(const ShotDesc& S, int x0, int y, int z, typename P::real r, int it,
+                                           int post) {
+    if (!row_updated<DIM, ORD>(S, y, z)) return;
+    const unsigned mask = chunk_mask<ORD>(S, x0);
+    if (!mask) return;
+    constexpr bool NC = read_only_loads<DIM, P, VPHASE>() && NCOK && !grouped<DIM, P, VPHASE>();
+    const cidx c = x0 + y * S.pitch + z * (cidx)S.plane;
+    // an indexed medium's tuple indices first: their load overlaps the field loads
+    unsigned ids = 0;
+    if (med_on<P>(S)) ids = med_ids(S, c);
+    const GlobalSrc<ORD, P, NC> src{S, c, x0};
+    chunk_work<DIM, ORD, P, VPHASE, NC, grouped<DIM, P, VPHASE>()>(S, src, c, x0, y, z, r, mask, ids, it, post);
 }
 
 // The (row, segment) units of tile (rb, sb) of shot S in one phase: the
