@@ -82,7 +82,7 @@ struct ShotDesc {
     double dtd;                   // DT (FP64)
     float inv_h;                  // 1/H (COMP16 multiplies; FP32/FP64 divide by H like the reference)
     float h;                      // H
-    double hd;
+    double hd, inv_hd;            // H, 1/H (FP64)
     void* f[BP_NFIELDS];          // field arrays (hi for COMP16)
     int8_t* flo[BP_NFIELDS];      // COMP16 residuals
     void* vc[VC_COUNT];

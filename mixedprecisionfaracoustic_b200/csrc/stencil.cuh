@@ -8,17 +8,85 @@
 
 namespace bpk {
 
+// Correctly rounded quotients without the divide routine's slow path.
+//
+// The compiler's IEEE division leaves its inline sequence for operands far from
+// 1, and a wavefield is full of them: ahead of the wavefront the scheme's own
+// domain of influence advances a cell per step, and its values fall off to
+// subnormal numbers, which then fill the grid out to the borders.  Here a tiny
+// dividend is scaled up by a power of two (exactly) and the quotient back down,
+// and the quotient is formed from the divisor's reciprocal y by two residual
+// corrections q += y (a - q b) with exact fused residuals (Markstein, IBM J.
+// Res. Dev. 34(1), 1990), which round correctly where nothing under- or
+// overflows.  A subnormal float result must not be rounded twice, so q is
+// first rounded to odd (Boldo and Melquiond, IEEE Trans. Comput. 57(4), 2008):
+// 24 bits to odd, then to at most 22 to nearest, is one rounding to nearest.
+// The binade below the smallest normal (23 bits) and quotients out of range
+// (infinite, NaN) take the division itself.  Equal to a / b bit for bit
+// (tests/test_gpu_quotient.py).
+template <class R> struct QuotRange;
+template <> struct QuotRange<float> {
+    static constexpr float small = 0x1p-30f, up = 0x1p64f, down = 0x1p-64f, lo = 0x1p-61f, hi = 0x1p120f;
+};
+template <> struct QuotRange<double> {
+    static constexpr double small = 0x1p-300, up = 0x1p600, down = 0x1p-600, lo = 0x1p-420, hi = 0x1p1000;
+};
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// a / b for y = 1 / b to within an ulp
+template <class R>
+__device__ __forceinline__ R quot_y(R a, R b, R y) {
+    using Q = QuotRange<R>;
+    const bool tiny = fabs(a) < Q::small;
+    const R t = mul_rn(a, tiny ? Q::up : (R)1);
+    R q = mul_rn(t, y);
+    q = fma_rn(fma_rn(-q, b, t), y, q);
+    q = fma_rn(fma_rn(-q, b, t), y, q);
+    if (fabs(q) >= Q::lo && fabs(q) < Q::hi) return mul_rn(q, tiny ? Q::down : (R)1);
+    if (a == (R)0) return mul_rn(a, b);            // the zero with the quotient's sign
+    if constexpr (sizeof(R) == 4) {
+        if (tiny && fabs(q) < 0x1p-63f) {
+            const float r = fma_rn(-q, b, t);      // a 2^64 - q b, exact
+            int w = __float_as_int(q);
+            if (r != 0.0f) w = (w + ((__float_as_int(r) ^ __float_as_int(b) ^ w) >> 31)) | 1;
+            return mul_rn(__int_as_float(w), Q::down);
+        }
+    }
+    return a / b;
+}
+// the reciprocal of b to within an ulp (0, infinite or NaN where b is out of range)
+__device__ __forceinline__ float recip(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return fma_rn(fma_rn(-b, y, 1.0f), y, y);
+}
+
+// num / c1 of the friction update.  FP32 through quot_y: 296 x 296 x 232 1194 ->
+// 1078 us per step, 4040 x 2040 165.9 -> 162.1 (B200, order 2).  CBF16 keeps the
+// division, which is the cheaper one where nothing is subnormal (4040 x 2040
+// 169.6 against 171.1), and so does FP64, whose exponents never run out.
+template <class P>
+__device__ __forceinline__ typename P::real quot(typename P::real a, typename P::real b) {
+    if constexpr (P::store == BP_PREC_FP32) return quot_y<float>(a, b, recip(b));
+    else return a == (typename P::real)0 ? a * b : a / b;
+}
+
 template <class P>
 __device__ __forceinline__ typename P::real deriv_div(typename P::real a, const ShotDesc& S) {
     // FP32: the reference divides by H.  q = a * (1/H) refined by one residual
     // step, q += (a - q H) * (1/H), with the exact fused residual a - q H,
     // matches the IEEE quotient a / H to within one ulp (equal in all but rare
     // near-tie cases) in 3 instructions instead of a full divide.
-    // FP64 divides; COMP16 (own arithmetic) multiplies by 1/H.  PolF32R takes
-    // the IEEE quotient like the reference; a zero dividend (the quiet grid
-    // ahead of the wavefront), which sends the divide routine down its slow
-    // path, gives the same signed zero as a product.
-    if constexpr (P::prec == BP_PREC_FP64) return a / (typename P::real)S.hd;
+    // FP64 takes the correctly rounded quotient (4040 x 2040: 653 -> 535 us per
+    // step against the division); COMP16 (own arithmetic) multiplies by 1/H.
+    // PolF32R takes the IEEE quotient like the reference (its inline sequence is
+    // the cheaper one there: 192^3 630 us per step, 673 with quot_y); a zero
+    // dividend (the quiet grid ahead of the wavefront), which sends the divide
+    // routine down its slow path, gives the same signed zero as a product.
+    if constexpr (P::prec == BP_PREC_FP64) return quot_y<double>(a, S.hd, S.inv_hd);
     else if constexpr (P::prec == BP_PREC_FP32 && P::exact) return a == 0.0f ? a * S.inv_h : __fdiv_rn(a, S.h);
     else if constexpr (P::prec == BP_PREC_FP32) {
         const float q = a * S.inv_h;
@@ -441,12 +509,8 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
                 nu[j] = uo + rho[j] * sum[j] - rr * (wn - wo);
             } else {
                 R wo = vw[j];
-                // IEEE division; a zero dividend (the whole quiet grid ahead of
-                // the wavefront) takes the divide routine's slow path, so its
-                // exact result, a zero with the quotient's sign, is formed by a
-                // product instead: 7-15 % off the V phase, bit-identical.
                 const R num = wo * c2[j] - S.dtr<R>() * (rf[j] * rho[j] * sum[j] + dp[j]);
-                const R wn = (c1[j] == (R)0) ? (R)0 : (num == (R)0 ? num * c1[j] : num / c1[j]);
+                const R wn = (c1[j] == (R)0) ? (R)0 : quot<P>(num, c1[j]);
                 nw[j] = wn;
                 nu[j] = vu[j] + S.dtr<R>() * rho[j] * sum[j] - rf[j] * rho[j] * (wn - wo);
             }
