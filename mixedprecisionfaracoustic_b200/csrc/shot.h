@@ -55,6 +55,10 @@ int inter_occupancy(int prec, int dim, int order, int rounding);
 cudaError_t launch_inter(int prec, int dim, int order, int rounding, const ShotDesc* d, int nshots, long long nitems,
                          int k, int post, int grid, unsigned long long* ctl, int* err, cudaStream_t st);
 int seg_cells();
+// COMP16 phase kernels (step_async.cu), behind launch_phase and phase_occupancy
+cudaError_t launch_phase_async(int dim, int order, bool v, const ShotDesc* d, int nshots, long long ntiles, int k,
+                               int grid, cudaStream_t st, int post);
+int phase_async_occupancy(int dim, int order, bool v);
 // TMA-staged 2D phase kernels (step_staged.cu)
 bool staged_supported(int prec, int dim);
 bool staged_default();           // whether BP_KERNEL_AUTO picks the staged kernels where supported

@@ -504,7 +504,9 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
                 // Half/main.cu:256-262 with Bt = (rhof rho^-1) Bp formed here
                 const R wo = RS ? mulr(vw[j], r) : vw[j], uo = RS ? mulr(vu[j], r) : vu[j];
                 R rr = rf[j] * rho[j];                    // rhof * rho^-1
-                R wn = c1[j] * wo - (rr * c2[j]) * sum[j] - c2[j] * dp[j];
+                // one contraction for every kernel family: the result must not
+                // depend on which products the compiler fuses here
+                const R wn = fma_rn(-c2[j], dp[j], fma_rn(c1[j], wo, -mul_rn(rr * c2[j], sum[j])));
                 nw[j] = wn;
                 nu[j] = uo + rho[j] * sum[j] - rr * (wn - wo);
             } else {
@@ -574,6 +576,12 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
 }
 
 // ---------------------------------------------------------------------------
+// COMP16's new normal stress.  c w, shared by the normal stresses, is rounded by
+// itself: written out, so that every kernel family stores the same bits.
+__device__ __forceinline__ float c16_normal(float o, float h2, float e2, float h, float e, float c, float w) {
+    return __fadd_rn(__fmaf_rn(h, e, __fmaf_rn(h2, e2, o)), __fmul_rn(c, w));
+}
+
 // Everything of the T phase after the velocity derivatives: masking, CPML
 // memory variables, the pressure and stress updates and their stores.  PRE:
 // the caller has already loaded the moduli and the old stresses into T, the
@@ -689,7 +697,7 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = oxx[j] + cH2[j] * (uyy[j] + uzz[j]) + cH[j] * uxx[j] + cC[j] * (wx[j] + wy[j] + wz[j]);
+                n[j] = c16_normal(oxx[j], cH2[j], (uyy[j] + uzz[j]), cH[j], uxx[j], cC[j], (wx[j] + wy[j] + wz[j]));
             else
                 n[j] = oxx[j] + dt * (cH2[j] * (uyy[j] + uzz[j]) + cH[j] * uxx[j] + cC[j] * (wx[j] + wy[j] + wz[j]));
         }
@@ -697,7 +705,7 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = oyy[j] + cH2[j] * (uxx[j] + uzz[j]) + cH[j] * uyy[j] + cC[j] * (wx[j] + wy[j] + wz[j]);
+                n[j] = c16_normal(oyy[j], cH2[j], (uxx[j] + uzz[j]), cH[j], uyy[j], cC[j], (wx[j] + wy[j] + wz[j]));
             else
                 n[j] = oyy[j] + dt * (cH2[j] * (uxx[j] + uzz[j]) + cH[j] * uyy[j] + cC[j] * (wx[j] + wy[j] + wz[j]));
         }
@@ -705,7 +713,7 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = ozz[j] + cH2[j] * (uxx[j] + uyy[j]) + cH[j] * uzz[j] + cC[j] * (wx[j] + wy[j] + wz[j]);
+                n[j] = c16_normal(ozz[j], cH2[j], (uxx[j] + uyy[j]), cH[j], uzz[j], cC[j], (wx[j] + wy[j] + wz[j]));
             else
                 n[j] = ozz[j] + dt * (cH2[j] * (uxx[j] + uyy[j]) + cH[j] * uzz[j] + cC[j] * (wx[j] + wy[j] + wz[j]));
         }
@@ -740,7 +748,7 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = oxx[j] + cH2[j] * uzz[j] + cH[j] * uxx[j] + cC[j] * (wx[j] + wz[j]);
+                n[j] = c16_normal(oxx[j], cH2[j], uzz[j], cH[j], uxx[j], cC[j], (wx[j] + wz[j]));
             else
                 n[j] = oxx[j] + dt * (cH2[j] * uzz[j] + cH[j] * uxx[j] + cC[j] * (wx[j] + wz[j]));
         }
@@ -748,7 +756,7 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = ozz[j] + cH2[j] * uxx[j] + cH[j] * uzz[j] + cC[j] * (wx[j] + wz[j]);
+                n[j] = c16_normal(ozz[j], cH2[j], uxx[j], cH[j], uzz[j], cC[j], (wx[j] + wz[j]));
             else
                 n[j] = ozz[j] + dt * (cH2[j] * uxx[j] + cH[j] * uzz[j] + cC[j] * (wx[j] + wz[j]));
         }

@@ -212,6 +212,8 @@ struct Launch {
     }
         if constexpr (P::graded) {           // the variable z grid: order 2 only
             BPK_LAUNCH(2, 2) BPK_LAUNCH(3, 2)
+        } else if constexpr (P::prec == BP_PREC_COMP16) {   // the others: step_async.cu
+            BPK_LAUNCH(3, 4)
         } else {
             BPK_LAUNCH(2, 2) BPK_LAUNCH(2, 4) BPK_LAUNCH(3, 2) BPK_LAUNCH(3, 4)
         }
@@ -224,6 +226,12 @@ struct Launch {
 
 // C++ entry points used by the host code (sim.cu, batch.cu).
 namespace bpk {
+// COMP16 phases that take the kernels of step_async.cu: all but 3D order 4,
+// whose 37 staged rows (15 KB a warp) leave too few warps on an SM: 240 x 230 x
+// 220 per-cell medium 1588 us per step staged, 1434 from the register tiles (140
+// x 130 x 120 uniform 262 and 280; B200).
+static bool c16_async(int dim, int order) { return dim == 2 || order == 2; }
+
 cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDesc* d_shots, int nshots,
                          long long ntiles, int k, int grid, cudaStream_t st, int post, int rounding, bool multi,
                          bool graded) {
@@ -235,6 +243,8 @@ cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDe
         return Launch<PolF32R>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
     if (prec == BP_PREC_FP32)
         return Launch<PolF32>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
+    if (prec == BP_PREC_COMP16 && c16_async(dim, order))
+        return launch_phase_async(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post);
     if (prec == BP_PREC_COMP16)
         return Launch<PolC16>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
     if (prec == BP_PREC_CBF16)
@@ -292,7 +302,8 @@ int phase_occupancy(int prec, int dim, int order, bool vphase, int rounding) {
     if (prec == BP_PREC_FP32 && rounding == BP_ROUND_REFERENCE) {
         BPK_FN(PolF32R, 2, 2) BPK_FN(PolF32R, 2, 4) BPK_FN(PolF32R, 3, 2) BPK_FN(PolF32R, 3, 4)
     } else if (prec == BP_PREC_FP32) { BPK_FN(PolF32, 2, 2) BPK_FN(PolF32, 2, 4) BPK_FN(PolF32, 3, 2) BPK_FN(PolF32, 3, 4) }
-    else if (prec == BP_PREC_COMP16) { BPK_FN(PolC16, 2, 2) BPK_FN(PolC16, 2, 4) BPK_FN(PolC16, 3, 2) BPK_FN(PolC16, 3, 4) }
+    else if (prec == BP_PREC_COMP16 && c16_async(dim, order)) return phase_async_occupancy(dim, order, vphase);
+    else if (prec == BP_PREC_COMP16) { BPK_FN(PolC16, 3, 4) }
     else if (prec == BP_PREC_CBF16) { BPK_FN(PolB24, 2, 2) BPK_FN(PolB24, 2, 4) BPK_FN(PolB24, 3, 2) BPK_FN(PolB24, 3, 4) }
     else { BPK_FN(PolF64, 2, 2) BPK_FN(PolF64, 2, 4) BPK_FN(PolF64, 3, 2) BPK_FN(PolF64, 3, 4) }
 #undef BPK_FN
@@ -323,14 +334,15 @@ static bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 // sharing the memory's fetch unit with other warps: 296 x 296 x 232 with a
 // per-cell medium reads 3.03 GB in the V phase without gaps, 2.57 GB with 80
 // chunks for 74, and takes 1435 -> 1190 (76) or 1267 (80) us per step; CBF16
-// there 1690 -> 1374 (80).  Gaps above 9 % cost more than they save (CBF16 140
-// x 130 x 120, 35 chunks: 208 us without, 228 at 40).  COMP16, bound by its
-// codec's instructions, takes no gaps (140 x 130 x 120: 233 against 296 us).
-static int row_chunks(int n, int prec) {
+// there 1690 -> 1374, COMP16 1323 -> 1287 (uniform, 80).  Gaps above 9 % cost
+// more than they save (CBF16 140 x 130 x 120, 35 chunks: 208 us without, 228 at
+// 40).  2D COMP16, bound by its codec's instructions, takes none (4040 x 2040:
+// 222 us without, 227 with).
+static int row_chunks(int n, int dim, int prec) {
     const int a64 = prec == BP_PREC_FP64 ? 2 : prec == BP_PREC_FP32 ? 4 : 8;
     auto up = [&](int a) { return (n + a - 1) / a * a; };
     if (prec == BP_PREC_FP32 && (up(2 * a64) - n) * 100 <= 6 * n) return up(2 * a64);
-    if (prec != BP_PREC_COMP16 && (up(a64) - n) * 100 <= 9 * n) return up(a64);
+    if ((dim == 3 || prec != BP_PREC_COMP16) && (up(a64) - n) * 100 <= 9 * n) return up(a64);
     return n;
 }
 
@@ -366,7 +378,7 @@ long long apply_tile_shape(ShotDesc& S, int dim, int prec, TileShape t) {
     const int ty = dim == 3 ? t.rows / t.tz : 1;
     S.nyb = dim == 3 ? (S.ny + ty - 1) / ty : 1;
     const long long blocks = dim == 3 ? (long long)S.nyb * ((S.nz + t.tz - 1) / t.tz) : (S.nrows + t.rows - 1) / t.rows;
-    S.cpr = row_chunks((S.nx + 3) / 4, prec);
+    S.cpr = row_chunks((S.nx + 3) / 4, dim, prec);
     magic_of(S.cpr, S.cpr_m, S.cpr_s);
     magic_of(S.nyb, S.nyb_m, S.nyb_s);
     S.nchunk_f = (int)(blocks * S.cpr);

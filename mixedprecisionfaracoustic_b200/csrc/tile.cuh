@@ -363,7 +363,7 @@ __device__ __forceinline__ void v_comp(const ShotDesc& S, const Src& src, cidx c
         if constexpr (P::prec == BP_PREC_COMP16) {
             const R wo = RS ? mulr(vw[j], r) : vw[j], uo = RS ? mulr(vu[j], r) : vu[j];
             R rr = rf[j] * rho[j];
-            R wn = c1[j] * wo - (rr * c2[j]) * sum[j] - c2[j] * dp[j];
+            const R wn = fma_rn(-c2[j], dp[j], fma_rn(c1[j], wo, -mul_rn(rr * c2[j], sum[j])));   // as v_tail
             nw[j] = wn;
             nu[j] = uo + rho[j] * sum[j] - rr * (wn - wo);
         } else {
@@ -509,12 +509,12 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, const Src& src, cid
     for (int j = 0; j < 4; j++) {
         if constexpr (DIM == 3) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = o[j] + cH2[j] * (uyy[j] + uzz[j]) + cH[j] * uxx[j] + cC[j] * (wx[j] + wy[j] + wz[j]);
+                n[j] = c16_normal(o[j], cH2[j], (uyy[j] + uzz[j]), cH[j], uxx[j], cC[j], (wx[j] + wy[j] + wz[j]));
             else
                 n[j] = o[j] + dt * (cH2[j] * (uyy[j] + uzz[j]) + cH[j] * uxx[j] + cC[j] * (wx[j] + wy[j] + wz[j]));
         } else {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = o[j] + cH2[j] * uzz[j] + cH[j] * uxx[j] + cC[j] * (wx[j] + wz[j]);
+                n[j] = c16_normal(o[j], cH2[j], uzz[j], cH[j], uxx[j], cC[j], (wx[j] + wz[j]));
             else
                 n[j] = o[j] + dt * (cH2[j] * uzz[j] + cH[j] * uxx[j] + cC[j] * (wx[j] + wz[j]));
         }
@@ -525,7 +525,7 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, const Src& src, cid
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = o[j] + cH2[j] * (uxx[j] + uzz[j]) + cH[j] * uyy[j] + cC[j] * (wx[j] + wy[j] + wz[j]);
+                n[j] = c16_normal(o[j], cH2[j], (uxx[j] + uzz[j]), cH[j], uyy[j], cC[j], (wx[j] + wy[j] + wz[j]));
             else
                 n[j] = o[j] + dt * (cH2[j] * (uxx[j] + uzz[j]) + cH[j] * uyy[j] + cC[j] * (wx[j] + wy[j] + wz[j]));
         }
@@ -536,12 +536,12 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, const Src& src, cid
     for (int j = 0; j < 4; j++) {
         if constexpr (DIM == 3) {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = o[j] + cH2[j] * (uxx[j] + uyy[j]) + cH[j] * uzz[j] + cC[j] * (wx[j] + wy[j] + wz[j]);
+                n[j] = c16_normal(o[j], cH2[j], (uxx[j] + uyy[j]), cH[j], uzz[j], cC[j], (wx[j] + wy[j] + wz[j]));
             else
                 n[j] = o[j] + dt * (cH2[j] * (uxx[j] + uyy[j]) + cH[j] * uzz[j] + cC[j] * (wx[j] + wy[j] + wz[j]));
         } else {
             if constexpr (P::prec == BP_PREC_COMP16)
-                n[j] = o[j] + cH2[j] * uxx[j] + cH[j] * uzz[j] + cC[j] * (wx[j] + wz[j]);
+                n[j] = c16_normal(o[j], cH2[j], uxx[j], cH[j], uzz[j], cC[j], (wx[j] + wz[j]));
             else
                 n[j] = o[j] + dt * (cH2[j] * uxx[j] + cH[j] * uzz[j] + cC[j] * (wx[j] + wz[j]));
         }
