@@ -82,7 +82,9 @@ struct ShotDesc {
     double dtd;                   // DT (FP64)
     float inv_h;                  // 1/H (COMP16 multiplies; FP32/FP64 divide by H like the reference)
     float h;                      // H
-    double hd, inv_hd;            // H, 1/H (FP64)
+    double hd, inv_hd, inv_hd_lo; // H, 1/H and its rest (FP64)
+    float inv_h_lo;               // the rest of 1/H (reference rounding)
+    int h_two_ops;                // a / H = fma(a, inv, a * lo) for every a (const_divisor, divisor.h)
     void* f[BP_NFIELDS];          // field arrays (hi for COMP16)
     int8_t* flo[BP_NFIELDS];      // COMP16 residuals
     void* vc[VC_COUNT];

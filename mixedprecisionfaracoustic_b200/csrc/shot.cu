@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "divisor.h"
 #include "shot.h"
 
 namespace bpk {
@@ -315,7 +316,9 @@ int Shot::create(const bp_config* c, const bp_medium* med, cudaStream_t st) {
         S.nzs_f = (p.nz - 2 * S.hw + S.zseg_f - 1) / S.zseg_f;
     }
     S.nt = c->nt;
-    S.dt = c->dt; S.dtd = c->dt; S.h = c->dx; S.hd = c->dx; S.inv_hd = 1.0 / S.hd; S.inv_h = 1.0f / c->dx;
+    S.dt = c->dt; S.dtd = c->dt; S.h = c->dx; S.hd = c->dx; S.inv_h = 1.0f / c->dx; S.inv_hd = 1.0 / S.hd;
+    S.h_two_ops = c->precision == BP_PREC_FP64 ? const_divisor(S.hd, S.inv_hd, &S.inv_hd_lo)
+                                               : const_divisor(S.h, S.inv_h, &S.inv_h_lo);
     for (int f = 0; f < BP_NFIELDS; f++) {
         S.f[f] = at(p.o_f[f]);
         S.flo[f] = (int8_t*)at(p.o_flo[f]);

@@ -74,21 +74,51 @@ __device__ __forceinline__ typename P::real quot(typename P::real a, typename P:
     else return a == (typename P::real)0 ? a * b : a / b;
 }
 
+// Differences divided by H with IEEE rounding: FP64 and the reference's rounding
+// (PolF32R).  H is one number, so 1/H is held as the unevaluated sum inv + lo
+// and a / H = fma(a, inv, a lo), two operations, correctly rounded for every a
+// where that holds for the H at hand (Brisebarre, Muller and Raina, IEEE Trans.
+// Comput. 53(8), 2004; const_divisor in divisor.h decides it exactly).  That
+// leaves out tiny and huge differences (and -0), the rim of the scheme's domain
+// of influence ahead of the wavefront: a chunk is differenced in two operations first,
+// and again through quot_y if any of its differences was one of those.  Measured
+// on B200 (us per step, once the field has spread / in the first 130 steps):
+// 192^3 reference rounding, order 2, 630 / 745 -> 404 / 585; 200 x 190 x 180 order
+// 4 698 / 914 -> 442 / 739; FP64 4040 x 2040 533 / 510 -> 408 / 376, 168^3 809 ->
+// 675.  One out-of-line call for the rim of each difference instead spilled
+// around the calls (FP64 168^3 1106, order 4 932).
+template <class P>
+__host__ __device__ constexpr bool two_op_policy() { return P::prec == BP_PREC_FP64 || P::exact; }
+// Q 0: the policy's own division; 1: two operations (false: not for this
+// difference); 2: quot_y
+template <class P, int Q>
+__device__ __forceinline__ bool deriv_q(typename P::real a, const ShotDesc& S, typename P::real& q) {
+    using R = typename P::real;
+    R h, inv, lo, least, most;
+    if constexpr (sizeof(R) == 8) { h = S.hd; inv = S.inv_hd; lo = S.inv_hd_lo; least = (R)0x1p-860; most = (R)0x1p900; }
+    else { h = S.h; inv = S.inv_h; lo = S.inv_h_lo; least = (R)0x1p-80f; most = (R)0x1p100f; }
+    if constexpr (Q == 2) {
+        q = quot_y<R>(a, h, inv);
+        return true;
+    } else {
+        q = fma_rn(a, inv, mul_rn(a, lo));        // +0 for +0 too
+        bool zero;
+        if constexpr (sizeof(R) == 8) zero = __double_as_longlong(a) == 0;
+        else zero = __float_as_int(a) == 0;
+        return (fabs(a) >= least && fabs(a) < most) || zero;
+    }
+}
+
 template <class P>
 __device__ __forceinline__ typename P::real deriv_div(typename P::real a, const ShotDesc& S) {
     // FP32: the reference divides by H.  q = a * (1/H) refined by one residual
     // step, q += (a - q H) * (1/H), with the exact fused residual a - q H,
     // matches the IEEE quotient a / H to within one ulp (equal in all but rare
     // near-tie cases) in 3 instructions instead of a full divide.
-    // FP64 takes the correctly rounded quotient (4040 x 2040: 653 -> 535 us per
-    // step against the division); COMP16 (own arithmetic) multiplies by 1/H.
-    // PolF32R takes the IEEE quotient like the reference (its inline sequence is
-    // the cheaper one there: 192^3 630 us per step, 673 with quot_y); a zero
-    // dividend (the quiet grid ahead of the wavefront), which sends the divide
-    // routine down its slow path, gives the same signed zero as a product.
-    if constexpr (P::prec == BP_PREC_FP64) return quot_y<double>(a, S.hd, S.inv_hd);
-    else if constexpr (P::prec == BP_PREC_FP32 && P::exact) return a == 0.0f ? a * S.inv_h : __fdiv_rn(a, S.h);
-    else if constexpr (P::prec == BP_PREC_FP32) {
+    // COMP16 (own arithmetic) multiplies by 1/H; FP64 and the reference's
+    // rounding go through deriv_q.
+    static_assert(!two_op_policy<P>(), "correctly rounded differences take deriv_q");
+    if constexpr (P::prec == BP_PREC_FP32) {
         const float q = a * S.inv_h;
         return __fmaf_rn(__fmaf_rn(-q, S.h, a), S.inv_h, q);
     } else return a * S.inv_h;

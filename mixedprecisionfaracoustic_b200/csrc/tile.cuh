@@ -6,6 +6,8 @@
 // Reference kernels: FD_V Float/main.cu:64-192, Half/main.cu:156-268; FD_T
 // Float/main.cu:194-295, Half/main.cu:270-371.
 #pragma once
+#include <type_traits>
+
 #include "post.cuh"
 #include "shot.h"
 
@@ -59,17 +61,12 @@ __device__ __forceinline__ int locate_shot(const ShotDesc* shots, int nshots, lo
 // (128 registers, no spills) now that a chunk's memory variables and
 // coefficients are loaded in batches: us per step on B200 at 3 -> 2 CTAs, 200^3
 // order 2 557 -> 417, order 4 588 -> 444, 104^3 order 4 123 -> 83, 140 x 130 x
-// 120 199 -> 147.  With the reference's rounding, whose divisions keep it busy
-// issuing, order 2 is fastest at 3 (192^3: 624 against 649 at 2), order 4 at 2
-// (200 x 190 x 180 per-cell medium: 747 -> 699).  COMP16, taken one output group
-// at a time (v_chunk_g/t_chunk_g, next to no spills), is fastest at 4 CTAs (64
-// registers) on the 552 x 552 x 424 and 200^3 grids; FP64 at 2 (128 registers;
-// uncapped it takes 196-240, one CTA per SM).
+// 120 199 -> 147, and 192^3 with the reference's rounding 525 -> 405.  COMP16
+// (order 4), taken one output group at a time (v_chunk_g/t_chunk_g, next to no
+// spills), is fastest at 4 CTAs (64 registers) on the 552 x 552 x 424 and 200^3
+// grids; FP64 at 2 (128 registers; uncapped it takes 196-240, one CTA per SM).
 #ifndef BP_MINB3_F32
 #define BP_MINB3_F32 2
-#endif
-#ifndef BP_MINB3_F32R
-#define BP_MINB3_F32R 3
 #endif
 #ifndef BP_MINB3_C16
 #define BP_MINB3_C16 4
@@ -91,7 +88,6 @@ __device__ __forceinline__ int locate_shot(const ShotDesc* shots, int nshots, lo
 template <int DIM, int ORD, class P, bool VPHASE>
 __host__ __device__ constexpr int phase_min_blocks() {
     if (P::store == BP_PREC_CBF16) return DIM == 3 ? BP_MINB3_B24 : (VPHASE ? BP_MINB_B24_V : BP_MINB_B24);
-    if (DIM == 3 && P::exact && ORD == 2) return BP_MINB3_F32R;
     if (DIM == 3) return P::prec == BP_PREC_FP32 ? BP_MINB3_F32 : P::prec == BP_PREC_COMP16 ? BP_MINB3_C16 : BP_MINB3_F64;
     return P::prec == BP_PREC_FP32 ? BP_MINB_F32
                                    : P::prec == BP_PREC_COMP16 ? (VPHASE ? BP_MINB_C16_V : BP_MINB_C16) : BP_MINB_F64;
@@ -151,29 +147,49 @@ struct GlobalSrc {
     }
 };
 
-// Difference along x of field F at the chunk (FWD: at x + 1/2), divided by H.
-template <int ORD, class P, int F, bool FWD, class Src>
-__device__ __forceinline__ void d_span(const ShotDesc& S, const Src& src, typename P::real (&d)[4]) {
+// Difference along x of field F at the chunk (FWD: at x + 1/2), divided by H as
+// deriv_q's Q says; false if that does not hold for one of the four.
+template <int ORD, class P, int F, bool FWD, int Q, class Src>
+__device__ __forceinline__ bool d_span(const ShotDesc& S, const Src& src, typename P::real (&d)[4]) {
     typename P::real v[4 + ORD];
     src.template span<F>(v);
+    bool ok = true;
 #pragma unroll
-    for (int j = 0; j < 4; j++) d[j] = deriv_div<P>(FWD ? dfwd<ORD>(v, j) : dbwd<ORD>(v, j), S);
+    for (int j = 0; j < 4; j++) {
+        const typename P::real q = FWD ? dfwd<ORD>(v, j) : dbwd<ORD>(v, j);
+        if constexpr (Q) ok = deriv_q<P, Q>(q, S, d[j]) && ok;
+        else d[j] = deriv_div<P>(q, S);
+    }
+    return ok;
 }
 // Difference across rows (AX 1: y, 2: z) of field F at the chunk, divided by
 // the spacing.
-template <int ORD, class P, int F, int AX, bool FWD, class Src>
-__device__ __forceinline__ void d_rows(const ShotDesc& S, const Src& src, int z, typename P::real (&d)[4]) {
+template <int ORD, class P, int F, int AX, bool FWD, int Q, class Src>
+__device__ __forceinline__ bool d_rows(const ShotDesc& S, const Src& src, int z, typename P::real (&d)[4]) {
     using R = typename P::real;
     R a[ORD + 1][4];
     src.template rows<F, AX>(a);
+    bool ok = true;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         R t[ORD + 1];
 #pragma unroll
         for (int k = 0; k <= ORD; k++) t[k] = a[k][j];
         const R q = FWD ? rfwd<ORD>(t) : rbwd<ORD>(t);
-        if constexpr (AX == 2) d[j] = deriv_z<P, FWD>(q, S, z);
+        if constexpr (Q) ok = deriv_q<P, Q>(q, S, d[j]) && ok;
+        else if constexpr (AX == 2) d[j] = deriv_z<P, FWD>(q, S, z);
         else d[j] = deriv_div<P>(q, S);
+    }
+    return ok;
+}
+// Runs differences(Q) for a chunk: as the policy divides, or in two operations
+// and, where these do not hold, again through quot_y.
+template <class P, class Fn>
+__device__ __forceinline__ void differences(const ShotDesc& S, const Fn& fn) {
+    if constexpr (two_op_policy<P>()) {
+        if (!S.h_two_ops || !fn(std::integral_constant<int, 1>{})) fn(std::integral_constant<int, 2>{});
+    } else {
+        fn(std::integral_constant<int, 0>{});
     }
 }
 
@@ -187,20 +203,25 @@ __device__ __forceinline__ void v_chunk(const ShotDesc& S, const Src& src, cidx 
     VState<typename P::real> V;
     V.mids = ids;
     // ---- derivatives of the old stresses (x1..s3, Float/main.cu:115-128) ----
-    d_span<ORD, P, BP_F_TXX, true>(S, src, V.x1);
-    d_span<ORD, P, BP_F_P, true>(S, src, V.s1);
-    d_span<ORD, P, BP_F_TXZ, false>(S, src, V.z2);
-    d_rows<ORD, P, BP_F_TXZ, 2, false>(S, src, z, V.x3);
-    d_rows<ORD, P, BP_F_TZZ, 2, true>(S, src, z, V.z1);
-    d_rows<ORD, P, BP_F_P, 2, true>(S, src, z, V.s3);
-    if constexpr (DIM == 3) {
-        d_span<ORD, P, BP_F_TXY, false>(S, src, V.y2);
-        d_rows<ORD, P, BP_F_TXY, 1, false>(S, src, z, V.x2);
-        d_rows<ORD, P, BP_F_TYY, 1, true>(S, src, z, V.y1);
-        d_rows<ORD, P, BP_F_TYZ, 2, false>(S, src, z, V.y3);
-        d_rows<ORD, P, BP_F_TYZ, 1, false>(S, src, z, V.z3);
-        d_rows<ORD, P, BP_F_P, 1, true>(S, src, z, V.s2);
-    }
+    differences<P>(S, [&](auto q) {
+        constexpr int Q = decltype(q)::value;
+        bool ok = true;
+        ok = d_span<ORD, P, BP_F_TXX, true, Q>(S, src, V.x1) && ok;
+        ok = d_span<ORD, P, BP_F_P, true, Q>(S, src, V.s1) && ok;
+        ok = d_span<ORD, P, BP_F_TXZ, false, Q>(S, src, V.z2) && ok;
+        ok = d_rows<ORD, P, BP_F_TXZ, 2, false, Q>(S, src, z, V.x3) && ok;
+        ok = d_rows<ORD, P, BP_F_TZZ, 2, true, Q>(S, src, z, V.z1) && ok;
+        ok = d_rows<ORD, P, BP_F_P, 2, true, Q>(S, src, z, V.s3) && ok;
+        if constexpr (DIM == 3) {
+            ok = d_span<ORD, P, BP_F_TXY, false, Q>(S, src, V.y2) && ok;
+            ok = d_rows<ORD, P, BP_F_TXY, 1, false, Q>(S, src, z, V.x2) && ok;
+            ok = d_rows<ORD, P, BP_F_TYY, 1, true, Q>(S, src, z, V.y1) && ok;
+            ok = d_rows<ORD, P, BP_F_TYZ, 2, false, Q>(S, src, z, V.y3) && ok;
+            ok = d_rows<ORD, P, BP_F_TYZ, 1, false, Q>(S, src, z, V.z3) && ok;
+            ok = d_rows<ORD, P, BP_F_P, 1, true, Q>(S, src, z, V.s2) && ok;
+        }
+        return ok;
+    });
     v_tail<DIM, ORD, P, false, RS, NC>(S, c, x0, y, z, r, mask, V, TailOut::v_of(S), src);
 }
 
@@ -211,20 +232,25 @@ __device__ __forceinline__ void t_chunk(const ShotDesc& S, const Src& src, cidx 
                                         typename P::real r, unsigned mask, unsigned ids) {
     TState<typename P::real> T;
     T.mids = ids;
-    d_span<ORD, P, BP_F_VUX, false>(S, src, T.uxx);
-    d_span<ORD, P, BP_F_VWX, false>(S, src, T.wx);
-    d_span<ORD, P, BP_F_VUZ, true>(S, src, T.uzx);
-    d_rows<ORD, P, BP_F_VUZ, 2, false>(S, src, z, T.uzz);
-    d_rows<ORD, P, BP_F_VWZ, 2, false>(S, src, z, T.wz);
-    d_rows<ORD, P, BP_F_VUX, 2, true>(S, src, z, T.uxz);
-    if constexpr (DIM == 3) {
-        d_span<ORD, P, BP_F_VUY, true>(S, src, T.uyx);
-        d_rows<ORD, P, BP_F_VUY, 1, false>(S, src, z, T.uyy);
-        d_rows<ORD, P, BP_F_VWY, 1, false>(S, src, z, T.wy);
-        d_rows<ORD, P, BP_F_VUX, 1, true>(S, src, z, T.uxy);
-        d_rows<ORD, P, BP_F_VUY, 2, true>(S, src, z, T.uyz);
-        d_rows<ORD, P, BP_F_VUZ, 1, true>(S, src, z, T.uzy);
-    }
+    differences<P>(S, [&](auto q) {
+        constexpr int Q = decltype(q)::value;
+        bool ok = true;
+        ok = d_span<ORD, P, BP_F_VUX, false, Q>(S, src, T.uxx) && ok;
+        ok = d_span<ORD, P, BP_F_VWX, false, Q>(S, src, T.wx) && ok;
+        ok = d_span<ORD, P, BP_F_VUZ, true, Q>(S, src, T.uzx) && ok;
+        ok = d_rows<ORD, P, BP_F_VUZ, 2, false, Q>(S, src, z, T.uzz) && ok;
+        ok = d_rows<ORD, P, BP_F_VWZ, 2, false, Q>(S, src, z, T.wz) && ok;
+        ok = d_rows<ORD, P, BP_F_VUX, 2, true, Q>(S, src, z, T.uxz) && ok;
+        if constexpr (DIM == 3) {
+            ok = d_span<ORD, P, BP_F_VUY, true, Q>(S, src, T.uyx) && ok;
+            ok = d_rows<ORD, P, BP_F_VUY, 1, false, Q>(S, src, z, T.uyy) && ok;
+            ok = d_rows<ORD, P, BP_F_VWY, 1, false, Q>(S, src, z, T.wy) && ok;
+            ok = d_rows<ORD, P, BP_F_VUX, 1, true, Q>(S, src, z, T.uxy) && ok;
+            ok = d_rows<ORD, P, BP_F_VUY, 2, true, Q>(S, src, z, T.uyz) && ok;
+            ok = d_rows<ORD, P, BP_F_VUZ, 1, true, Q>(S, src, z, T.uzy) && ok;
+        }
+        return ok;
+    });
     t_tail<DIM, ORD, P, false, RS, NC>(S, c, x0, y, z, r, mask, T, TailOut::t_of(S), src);
 }
 
@@ -297,22 +323,27 @@ __device__ __forceinline__ void v_comp(const ShotDesc& S, const Src& src, cidx c
     // dx, dy, dz: the stress derivatives summed into this component (dy in 3D
     // only); dp: the pressure derivative along AX.  Slots as in v_tail.
     R dx[4], dy[4], dz[4], dp[4];
-    if constexpr (AX == 0) {
-        d_span<ORD, P, BP_F_TXX, true>(S, src, dx);                          // x1
-        if constexpr (DIM == 3) d_rows<ORD, P, BP_F_TXY, 1, false>(S, src, z, dy);   // x2
-        d_rows<ORD, P, BP_F_TXZ, 2, false>(S, src, z, dz);                           // x3
-        d_span<ORD, P, BP_F_P, true>(S, src, dp);                            // s1
-    } else if constexpr (AX == 1) {
-        d_span<ORD, P, BP_F_TXY, false>(S, src, dx);                         // y2
-        d_rows<ORD, P, BP_F_TYY, 1, true>(S, src, z, dy);                            // y1
-        d_rows<ORD, P, BP_F_TYZ, 2, false>(S, src, z, dz);                           // y3
-        d_rows<ORD, P, BP_F_P, 1, true>(S, src, z, dp);                              // s2
-    } else {
-        d_span<ORD, P, BP_F_TXZ, false>(S, src, dx);                         // z2
-        if constexpr (DIM == 3) d_rows<ORD, P, BP_F_TYZ, 1, false>(S, src, z, dy);   // z3
-        d_rows<ORD, P, BP_F_TZZ, 2, true>(S, src, z, dz);                            // z1
-        d_rows<ORD, P, BP_F_P, 2, true>(S, src, z, dp);                              // s3
-    }
+    differences<P>(S, [&](auto q) {
+        constexpr int Q = decltype(q)::value;
+        bool ok = true;
+        if constexpr (AX == 0) {
+            ok = d_span<ORD, P, BP_F_TXX, true, Q>(S, src, dx) && ok;                          // x1
+            if constexpr (DIM == 3) ok = d_rows<ORD, P, BP_F_TXY, 1, false, Q>(S, src, z, dy) && ok;   // x2
+            ok = d_rows<ORD, P, BP_F_TXZ, 2, false, Q>(S, src, z, dz) && ok;                           // x3
+            ok = d_span<ORD, P, BP_F_P, true, Q>(S, src, dp) && ok;                            // s1
+        } else if constexpr (AX == 1) {
+            ok = d_span<ORD, P, BP_F_TXY, false, Q>(S, src, dx) && ok;                         // y2
+            ok = d_rows<ORD, P, BP_F_TYY, 1, true, Q>(S, src, z, dy) && ok;                            // y1
+            ok = d_rows<ORD, P, BP_F_TYZ, 2, false, Q>(S, src, z, dz) && ok;                           // y3
+            ok = d_rows<ORD, P, BP_F_P, 1, true, Q>(S, src, z, dp) && ok;                              // s2
+        } else {
+            ok = d_span<ORD, P, BP_F_TXZ, false, Q>(S, src, dx) && ok;                         // z2
+            if constexpr (DIM == 3) ok = d_rows<ORD, P, BP_F_TYZ, 1, false, Q>(S, src, z, dy) && ok;   // z3
+            ok = d_rows<ORD, P, BP_F_TZZ, 2, true, Q>(S, src, z, dz) && ok;                            // z1
+            ok = d_rows<ORD, P, BP_F_P, 2, true, Q>(S, src, z, dp) && ok;                              // s3
+        }
+        return ok;
+    });
     if constexpr (P::prec == BP_PREC_COMP16 && RS) {
         scale4(dx, r); scale4(dz, r); scale4(dp, r);
         if constexpr (DIM == 3) scale4(dy, r);
@@ -411,16 +442,21 @@ __device__ __forceinline__ void t_shear(const ShotDesc& S, const Src& src, cidx 
                                         typename P::real r, unsigned mask, unsigned ids, void* const (&psi)[3]) {
     using R = typename P::real;
     R a[4], b[4];    // the two derivatives, in the order of the update's sum
-    if constexpr (SH == 0) {
-        d_rows<ORD, P, BP_F_VUX, 1, true>(S, src, z, a);        // uxy
-        d_span<ORD, P, BP_F_VUY, true>(S, src, b);      // uyx
-    } else if constexpr (SH == 1) {
-        d_rows<ORD, P, BP_F_VUY, 2, true>(S, src, z, a);        // uyz
-        d_rows<ORD, P, BP_F_VUZ, 1, true>(S, src, z, b);        // uzy
-    } else {
-        d_rows<ORD, P, BP_F_VUX, 2, true>(S, src, z, a);        // uxz
-        d_span<ORD, P, BP_F_VUZ, true>(S, src, b);      // uzx
-    }
+    differences<P>(S, [&](auto q) {
+        constexpr int Q = decltype(q)::value;
+        bool ok = true;
+        if constexpr (SH == 0) {
+            ok = d_rows<ORD, P, BP_F_VUX, 1, true, Q>(S, src, z, a) && ok;        // uxy
+            ok = d_span<ORD, P, BP_F_VUY, true, Q>(S, src, b) && ok;      // uyx
+        } else if constexpr (SH == 1) {
+            ok = d_rows<ORD, P, BP_F_VUY, 2, true, Q>(S, src, z, a) && ok;        // uyz
+            ok = d_rows<ORD, P, BP_F_VUZ, 1, true, Q>(S, src, z, b) && ok;        // uzy
+        } else {
+            ok = d_rows<ORD, P, BP_F_VUX, 2, true, Q>(S, src, z, a) && ok;        // uxz
+            ok = d_span<ORD, P, BP_F_VUZ, true, Q>(S, src, b) && ok;      // uzx
+        }
+        return ok;
+    });
     mask0(a, mask); mask0(b, mask);
     if constexpr (SH == 0) {
         cpml_g<DIM, RS, typename P::real, P::exact>(S, psi, 0, 3, true, slab_index(S, 0, x0, y, z), x0, y, z, b, r);
@@ -459,14 +495,19 @@ __device__ __forceinline__ void t_chunk_g(const ShotDesc& S, const Src& src, cid
 
     // normal stresses and pressure: the divergence derivatives (uyy, wy in 3D)
     R uxx[4], uyy[4], uzz[4], wx[4], wy[4], wz[4];
-    d_span<ORD, P, BP_F_VUX, false>(S, src, uxx);
-    d_span<ORD, P, BP_F_VWX, false>(S, src, wx);
-    if constexpr (DIM == 3) {
-        d_rows<ORD, P, BP_F_VUY, 1, false>(S, src, z, uyy);
-        d_rows<ORD, P, BP_F_VWY, 1, false>(S, src, z, wy);
-    }
-    d_rows<ORD, P, BP_F_VUZ, 2, false>(S, src, z, uzz);
-    d_rows<ORD, P, BP_F_VWZ, 2, false>(S, src, z, wz);
+    differences<P>(S, [&](auto q) {
+        constexpr int Q = decltype(q)::value;
+        bool ok = true;
+        ok = d_span<ORD, P, BP_F_VUX, false, Q>(S, src, uxx) && ok;
+        ok = d_span<ORD, P, BP_F_VWX, false, Q>(S, src, wx) && ok;
+        if constexpr (DIM == 3) {
+            ok = d_rows<ORD, P, BP_F_VUY, 1, false, Q>(S, src, z, uyy) && ok;
+            ok = d_rows<ORD, P, BP_F_VWY, 1, false, Q>(S, src, z, wy) && ok;
+        }
+        ok = d_rows<ORD, P, BP_F_VUZ, 2, false, Q>(S, src, z, uzz) && ok;
+        ok = d_rows<ORD, P, BP_F_VWZ, 2, false, Q>(S, src, z, wz) && ok;
+        return ok;
+    });
     mask0(uxx, mask); mask0(wx, mask); mask0(uzz, mask); mask0(wz, mask);
     if constexpr (DIM == 3) { mask0(uyy, mask); mask0(wy, mask); }
     {

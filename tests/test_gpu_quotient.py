@@ -59,3 +59,25 @@ def test_quotients_equal_the_division(tmp_path):
     r = subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=300)
     rows = [tuple(map(int, line.split())) for line in r.stdout.splitlines()]
     assert rows == [(m, 0, 0) for m in range(4)]
+
+
+@pytest.mark.parametrize("dx", [5.0, 5.02465773, 4.0])
+@pytest.mark.parametrize("order", [2, 4])
+def test_reference_rounding_at_spacings_of_each_kind(dx, order):
+    """A spacing the two-operation division holds for, one it does not (every
+    difference through quot_y), and a power of two: against the oracle's
+    reference arithmetic, <= 1e-5 as everywhere (test_gpu_parity.py)."""
+    import numpy as np
+    from mixedprecisionfaracoustic_b200 import Simulation
+    from oracle import oracle as O
+    from test_gpu_parity import small_2d
+    cfg, med = small_2d(order, "fp32", nx=90, nz=61, nt=200)
+    cfg.dx, cfg.rounding = dx, "reference"
+    with Simulation(cfg, med) as s:
+        s.run(cfg.nt)
+        got = {c: s.traces(c) for c in ("txx", "vux", "p")}
+    o = O.Oracle(cfg, med, O.REF32)
+    o.run(cfg.nt)
+    for c, g in got.items():
+        want = np.asarray(o.traces(c), np.float64)
+        assert np.linalg.norm(g - want) <= 1e-5 * np.linalg.norm(want), c
