@@ -87,7 +87,11 @@ int BatchCore::rebuild() {
     run.variant = kernel;
     run.multi_unit = ts.rows * ts.segs > phase_threads() / 32;
     run.indexed = false;
-    for (int i = 0; i < n; i++) run.indexed = run.indexed || shots[i]->med_tuples > 0;
+    run.all_indexed = true;
+    for (int i = 0; i < n; i++) {
+        run.indexed = run.indexed || shots[i]->med_tuples > 0;
+        run.all_indexed = run.all_indexed && shots[i]->med_tuples > 0;
+    }
     run.configure(prec, dim, order, d_descs, n, t0, t0s, t0m, maxrec, st, ctas_per_sm,
                   steps_per_sync > 0 ? steps_per_sync : 32);
     return BP_OK;

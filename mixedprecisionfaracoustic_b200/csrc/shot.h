@@ -15,10 +15,11 @@ namespace bpk {
 // post = 1: the T phase also records the receivers and injects the next source
 // sample (every receiver and the source lie in cells the T phase visits)
 // rounding = BP_ROUND_REFERENCE (FP32): the PolF32R instantiation; multi: the
-// tile shape has more (row, segment) units than a CTA has warps
+// tile shape has more (row, segment) units than a CTA has warps; indexed: every
+// shot reads an indexed medium
 cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDesc* d_shots, int nshots,
                          long long ntiles, int k, int grid, cudaStream_t st, int post = 0, int rounding = 0,
-                         bool multi = false, bool graded = false);
+                         bool multi = false, bool graded = false, bool indexed = false);
 cudaError_t launch_post(int prec, const ShotDesc* d_shots, int nshots, int max_rec, int k, int do_record,
                         cudaStream_t st);
 cudaError_t launch_inject(int prec, const ShotDesc* d_shots, int nshots, int k, cudaStream_t st);

@@ -747,4 +747,21 @@ __device__ __forceinline__ void flat_units(const ShotDesc& S, int lt, int warp, 
     }
 }
 
+// L2 prefetch of this warp's unit of tile lt: the FP32 fields, a 128-byte line
+// of one array per lane (no registers held, nothing waited for).
+template <int DIM>
+__device__ __forceinline__ void flat_prefetch(const ShotDesc& S, int lt, int warp, int lane) {
+    const int lr = S.tile_lr;
+    const int q = (((lt << S.tile_ls) + (warp >> lr)) << 5) + (lane & 3) * 8;
+    int x0, y, z;
+    if (!flat_cell<DIM>(S, q, warp & ((1 << lr) - 1), x0, y, z)) return;
+    const cidx c = x0 + y * S.pitch + z * (cidx)S.plane;
+#pragma unroll
+    for (int f = 0; f < BP_NFIELDS; f += 8) {
+        const int a = f + (lane >> 2);
+        if (a < BP_NFIELDS && S.f[a])
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const float*>(S.f[a]) + c));
+    }
+}
+
 }  // namespace bpk
