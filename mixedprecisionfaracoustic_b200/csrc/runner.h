@@ -33,6 +33,7 @@ struct Runner {
     int rounding = BP_ROUND_FAST;      // FP32 BP_ROUND_REFERENCE: PolF32R register kernels only
     bool multi_unit = false;           // the shots' tile shape has more units than a CTA has warps
     bool indexed = false;              // some shot reads an indexed medium (not the marching or staged kernels)
+    const ShotDesc* one = nullptr;     // a single shot's descriptor on the host (bp_sim)
     bool all_indexed = false;          // every shot does
     bool graded = false;               // a variable z grid (PolF32G register kernels only)
     long long ntiles_f = 0;            // tasks of the fused step kernel (0: some shot cannot take it)
@@ -53,7 +54,8 @@ struct Runner {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int ov = phase_occupancy(prec, dim, order, true, rounding), ot = phase_occupancy(prec, dim, order, false, rounding);
+        int ov = phase_occupancy(prec, dim, order, true, rounding, indexed_form()),
+            ot = phase_occupancy(prec, dim, order, false, rounding, indexed_form());
         if (ctas_per_sm > 0) { ov = ov < ctas_per_sm ? ov : ctas_per_sm; ot = ot < ctas_per_sm ? ot : ctas_per_sm; }
         long long gv = (long long)ov * sms, gt = (long long)ot * sms;
         grid_v = (int)(gv < tiles ? gv : (tiles > 0 ? tiles : 1));
@@ -115,13 +117,20 @@ struct Runner {
 #endif
         return post_in_t && !march && !staged;
     }
+    // Whether the phases run as for an indexed medium.  2D order-2 COMP16 launches
+    // of per-cell media take their own shape (AsyncShape, step_async.cu) from 8
+    // tiles a CTA on: 4040 x 2040 262 -> 235 us per step, 817 x 1073 30.7 -> 32.9;
+    // order 4 loses by it (292 -> 358)
+    bool indexed_form() const {
+        return all_indexed || (prec == BP_PREC_COMP16 && !(dim == 2 && order == 2 && ntiles >= 8LL * 3 * 148));
+    }
     // launches of one step of the two-phase kernels
     int launches_per_step() const { return fused_post() ? 2 : 3; }
     cudaError_t phase(bool v, int k) {
         if (march) return launch_phase_march(prec, order, v, d_shots, nshots, ntiles_m, k, st);
         if (staged) return launch_phase_staged(prec, order, v, d_shots, nshots, ntiles_s, k, grid_s, d_err, st);
         return launch_phase(prec, dim, order, v, d_shots, nshots, ntiles, k, v ? grid_v : grid_t, st,
-                            (!v && fused_post()) ? 1 : 0, rounding, multi_unit, graded, all_indexed);
+                            (!v && fused_post()) ? 1 : 0, rounding, multi_unit, graded, indexed_form(), one);
     }
 
     // One step (index k of the chunk) of the two-phase kernels, or of the

@@ -150,6 +150,7 @@ int bp_create(const bp_config* cfg, const bp_medium* medium, bp_sim** out) {
     s->run.rounding = cfg->rounding;
     s->run.ntiles_f = s->shot.ntiles_f;
     s->run.nitems_i = s->shot.nitems_i;
+    s->run.one = &s->shot.desc;
     s->run.indexed = s->run.all_indexed = s->shot.med_tuples > 0;
     s->run.nbands_i = s->shot.desc.nbands_i;
     s->run.configure(cfg->precision, cfg->dim, cfg->order, s->shot.d_desc, 1, s->shot.ntiles, s->shot.ntiles_s,
