@@ -29,8 +29,11 @@ bool const_divisor(R h, R inv, R* lo) {
     const uint64_t B = (uint64_t)std::ldexp(f, p);
     int s = 0;
     while (!((B >> s) & 1)) s++;
+    // No J below is a multiple of 8.  That covers powers of two and every double
+    // widened from a float (s >= 29), for which the search would otherwise take
+    // steps of Bo <= 2^24 through 2^52 dividends.
+    if (s > 2) return true;
     const uint64_t Bo = B >> s;
-    if (Bo == 1) return true;                        // a power of two: lo = 0 and inv is exact
     const auto mul = [&](uint64_t x, uint64_t y) { return (uint64_t)((u128)x * y % Bo); };
     const auto wrong = [&](uint64_t A) {
         volatile R a = (R)A, t = a * *lo, q = std::fma((R)a, inv, (R)t), d = a / h;
