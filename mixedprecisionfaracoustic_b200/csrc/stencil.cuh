@@ -65,12 +65,18 @@ __device__ __forceinline__ float recip(float b) {
 }
 
 // num / c1 of the friction update.  FP32 through quot_y: 296 x 296 x 232 1194 ->
-// 1078 us per step, 4040 x 2040 165.9 -> 162.1 (B200, order 2).  CBF16 keeps the
-// division, which is the cheaper one where nothing is subnormal (4040 x 2040
-// 169.6 against 171.1), and so does FP64, whose exponents never run out.
-template <class P>
+// 1078 us per step, 4040 x 2040 165.9 -> 162.1 (B200, order 2).  CBF16 in 2D too,
+// after a test for zero, which is what the quiet grid ahead of the domain of
+// influence divides: the 4040 x 2040 layered run of 8000 steps, 180.3 us per
+// step with the division (158 early, 192 late), 169.1 without the test (164,
+// 175), 165.1 with it (156, 175); order 4 201.7, 190.5 and 186.0; 817 x 1073 at
+// step 1500 24.0, 22.3 and 22.0.  In 3D CBF16 keeps the division: 200 x 190 x 180
+// 367 against 376 at step 600, 296 x 296 x 232 965 against 975 early, though 1208
+// against 1092 late.  So does FP64, whose exponents never run out.
+template <class P, int DIM>
 __device__ __forceinline__ typename P::real quot(typename P::real a, typename P::real b) {
     if constexpr (P::store == BP_PREC_FP32) return quot_y<float>(a, b, recip(b));
+    else if constexpr (P::store == BP_PREC_CBF16 && DIM == 2) return a == 0.0f ? a * b : quot_y<float>(a, b, recip(b));
     else return a == (typename P::real)0 ? a * b : a / b;
 }
 
@@ -542,7 +548,7 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
             } else {
                 R wo = vw[j];
                 const R num = wo * c2[j] - S.dtr<R>() * (rf[j] * rho[j] * sum[j] + dp[j]);
-                const R wn = (c1[j] == (R)0) ? (R)0 : quot<P>(num, c1[j]);
+                const R wn = (c1[j] == (R)0) ? (R)0 : quot<P, DIM>(num, c1[j]);
                 nw[j] = wn;
                 nu[j] = vu[j] + S.dtr<R>() * rho[j] * sum[j] - rf[j] * rho[j] * (wn - wo);
             }

@@ -402,7 +402,7 @@ __device__ __forceinline__ void v_comp(const ShotDesc& S, const Src& src, cidx c
         } else {
             R wo = vw[j];
             const R num = wo * c2[j] - S.dtr<R>() * (rf[j] * rho[j] * sum[j] + dp[j]);
-            const R wn = (c1[j] == (R)0) ? (R)0 : quot<P>(num, c1[j]);
+            const R wn = (c1[j] == (R)0) ? (R)0 : quot<P, DIM>(num, c1[j]);
             nw[j] = wn;
             nu[j] = vu[j] + S.dtr<R>() * rho[j] * sum[j] - rf[j] * rho[j] * (wn - wo);
         }
