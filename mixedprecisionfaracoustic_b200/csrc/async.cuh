@@ -99,13 +99,14 @@ __device__ __forceinline__ void slot_fill(const ShotDesc& S, char* slot, int e, 
 
 // Source of a chunk's field values (tile.cuh) over the warp's slots.
 template <int DIM, int ORD, class P, bool V>
-struct AsyncSrc {
+struct AsyncSrc : SrcForm {
     static_assert(P::store == BP_PREC_COMP16, "the slots hold COMP16 chunks");
     using R = typename P::real;
     static constexpr SlotTable T = slot_table<DIM, ORD, V>();
     static constexpr int kBytes = T.n * kSlotBytes;
     char* w;          // the warp's slots
     int lane;
+    __device__ __forceinline__ AsyncSrc(char* w_, int lane_) : w(w_), lane(lane_) {}
 
     template <int I>
     __device__ __forceinline__ void get4(R (&v)[4]) const {

@@ -73,10 +73,12 @@ __device__ __forceinline__ float recip(float b) {
 // step 1500 24.0, 22.3 and 22.0.  In 3D CBF16 keeps the division: 200 x 190 x 180
 // 367 against 376 at step 600, 296 x 296 x 232 965 against 975 early, though 1208
 // against 1092 late.  So does FP64, whose exponents never run out.
-template <class P, int DIM>
+// TEST0: FP32 tests for zero as well (SrcForm).
+template <class P, int DIM, bool TEST0 = false>
 __device__ __forceinline__ typename P::real quot(typename P::real a, typename P::real b) {
-    if constexpr (P::store == BP_PREC_FP32) return quot_y<float>(a, b, recip(b));
-    else if constexpr (P::store == BP_PREC_CBF16 && DIM == 2) return a == 0.0f ? a * b : quot_y<float>(a, b, recip(b));
+    if constexpr (P::store == BP_PREC_FP32 && !TEST0) return quot_y<float>(a, b, recip(b));
+    else if constexpr (P::store == BP_PREC_FP32 || (P::store == BP_PREC_CBF16 && DIM == 2))
+        return a == 0.0f ? a * b : quot_y<float>(a, b, recip(b));
     else return a == (typename P::real)0 ? a * b : a / b;
 }
 
@@ -313,10 +315,17 @@ __device__ __forceinline__ void cpml_slot(R (&d)[4], void* base, long long cells
 // us per step, slot by slot -> at once (FP32 where not named): 296 x 296 x 232
 // 1740 -> 1553, 4040 x 2040 179 -> 166, 817 x 1073 21.2 -> 19.3, 200^3 order 2
 // 492 -> 482; FP64 1040 x 540 40.0 -> 38.1.
-template <int NS, bool RS, class R, bool EX = false>
+template <int NS, bool RS, class R, bool EX = false, bool SLOTWISE = false>
 __device__ __forceinline__ void cpml_axis(R (*const (&d)[NS])[4], unsigned half, void* base, long long cells,
                                           cidx sidx, bool xaxis, int pos, int x0, const void* pb, const void* pe,
                                           const void* pb2, const void* pe2, R r, void* out, bool st) {
+    if constexpr (SLOTWISE) {
+#pragma unroll
+        for (int k = 0; k < NS; k++)
+            cpml_slot<NS, RS, R, EX>(*d[k], base, cells, k, sidx, xaxis, pos, x0, (half >> k & 1) ? pb2 : pb,
+                                     (half >> k & 1) ? pe2 : pe, r, out, st);
+        return;
+    }
     R ps[NS][4], pv[NS][4];
 #pragma unroll
     for (int k = 0; k < NS; k++) {
@@ -421,11 +430,21 @@ __device__ __forceinline__ void tcoef4(const ShotDesc& S, int k, cidx c, unsigne
     P::template ld4<NC>(S.tc[k], S.tclo[k], c, o);
 }
 
+// How the tails load what they need besides the derivatives, by where a chunk's
+// values come from (the sources below and in tile.cuh and async.cuh).  kAhead: FP32
+// loads every axis' coefficients and old velocities before the first axis'
+// stores, and divides without a test for zero.  kSlotwise: the CPML memory
+// variables slot by slot.
+struct SrcForm {
+    static constexpr bool kAhead = true, kSlotwise = false;
+};
+
 // The chunk's old values of a field the phase updates, from its array.
 template <class P>
-struct ArraySrc {
+struct ArraySrc : SrcForm {
     const ShotDesc& S;
     cidx c;
+    __device__ __forceinline__ ArraySrc(const ShotDesc& S_, cidx c_) : S(S_), c(c_) {}
     template <int F>
     __device__ __forceinline__ void own(typename P::real (&v)[4]) const { P::ld4(S.f[F], S.flo[F], c, v); }
 };
@@ -504,7 +523,7 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
         auto axis = [&](R (*const (&d)[NS])[4], unsigned half, int a, int pos) {
             const cidx si = slab_index(S, a, x0, y, z);
             if (si >= 0)
-                cpml_axis<NS, RS, R, P::exact>(d, half, O.psi_in[a], S.slab_cells[a], si, a == 0, pos, x0, S.pb[a],
+                cpml_axis<NS, RS, R, P::exact, Src::kSlotwise>(d, half, O.psi_in[a], S.slab_cells[a], si, a == 0, pos, x0, S.pb[a],
                                                S.pe[a], S.pb2[a], S.pe2[a], r, O.psi_out ? O.psi_out[a] : nullptr, O.store);
         };
         if constexpr (DIM == 3) {
@@ -554,7 +573,7 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
             } else {
                 R wo = vw[j];
                 const R num = wo * c2[j] - S.dtr<R>() * (rf[j] * rho[j] * sum[j] + dp[j]);
-                const R wn = (c1[j] == (R)0) ? (R)0 : quot<P, DIM>(num, c1[j]);
+                const R wn = (c1[j] == (R)0) ? (R)0 : quot<P, DIM, !Src::kAhead>(num, c1[j]);
                 nw[j] = wn;
                 nu[j] = vu[j] + S.dtr<R>() * rho[j] * sum[j] - rf[j] * rho[j] * (wn - wo);
             }
@@ -571,7 +590,7 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
     // 1436, 4040 x 2040 per-cell 205.8 -> 202.9, indexed 162.6 -> 163.4.  The
     // 3-byte and FP64 forms spill and lose: COMP16 2D 259 -> 321, CBF16 296 x
     // 296 x 232 1681 -> 1791, FP64 168^3 814 -> 899.
-    constexpr bool kAhead = P::store == BP_PREC_FP32;
+    constexpr bool kAhead = P::store == BP_PREC_FP32 && Src::kAhead;
     auto load_x = [&] {
         if (!med) P::template ld4<NC>(S.vc[VC_RHOF], S.vclo[VC_RHOF], c, rf);   // indexed: with the x group
         load_axis(VC_RHO_X, VC_CC1_X, VC_CC2_X, rho_x, c1_x, c2_x);
@@ -609,12 +628,12 @@ __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y,
 template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
 __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
                                        unsigned mask, VState<typename P::real>& V) {
-    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, TailOut::v_of(S), ArraySrc<P>{S, c});
+    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, TailOut::v_of(S), ArraySrc<P>(S, c));
 }
 template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
 __device__ __forceinline__ void v_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
                                        unsigned mask, VState<typename P::real>& V, const TailOut& O) {
-    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, O, ArraySrc<P>{S, c});
+    v_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, V, O, ArraySrc<P>(S, c));
 }
 
 // ---------------------------------------------------------------------------
@@ -697,7 +716,7 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
         auto axis = [&](R (*const (&d)[NS])[4], unsigned half, int a, int pos) {
             const cidx si = slab_index(S, a, x0, y, z);
             if (si >= 0)
-                cpml_axis<NS, RS, R, P::exact>(d, half, O.psi_in[a], S.slab_cells[a], si, a == 0, pos, x0, S.pb[a],
+                cpml_axis<NS, RS, R, P::exact, Src::kSlotwise>(d, half, O.psi_in[a], S.slab_cells[a], si, a == 0, pos, x0, S.pb[a],
                                                S.pe[a], S.pb2[a], S.pe2[a], r, nullptr, O.store);
         };
         if constexpr (DIM == 3) {
@@ -815,12 +834,12 @@ __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y,
 template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
 __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
                                        unsigned mask, TState<typename P::real>& T) {
-    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, TailOut::t_of(S), ArraySrc<P>{S, c});
+    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, TailOut::t_of(S), ArraySrc<P>(S, c));
 }
 template <int DIM, int ORD, class P, bool PRE, bool RS, bool NC = kReadOnlyPath>
 __device__ __forceinline__ void t_tail(const ShotDesc& S, cidx c, int x0, int y, int z, typename P::real r,
                                        unsigned mask, TState<typename P::real>& T, const TailOut& O) {
-    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, O, ArraySrc<P>{S, c});
+    t_tail<DIM, ORD, P, PRE, RS, NC>(S, c, x0, y, z, r, mask, T, O, ArraySrc<P>(S, c));
 }
 
 }  // namespace bpk

@@ -58,7 +58,7 @@ __device__ __forceinline__ void async_units(const ShotDesc& S, char* mine, int l
         __syncwarp();
         const unsigned mask = on ? chunk_mask<ORD>(S, x0) : 0;
         if (mask) {
-            const Src src{mine, lane};
+            const Src src(mine, lane);
             chunk_work<DIM, ORD, P, VPHASE, false, false>(S, src, c, x0, y, z, r, mask, ids, it, post);
         }
         __syncwarp();                     // every lane has read before the slots are filled again

@@ -100,6 +100,16 @@ __device__ __forceinline__ void span_of(const typename P::real (&c)[4], const Ed
     }
 }
 
+// The tails' loads: at 64 registers what is loaded ahead spills (4040 x 2040
+// layered FP32 292 us per step with the coefficients ahead, 265 without; order 4
+// 372 and 326), and so do COMP16's memory variables at order 4 (609, slot by slot
+// 573; order 2 430 and 437; B200).
+template <int ORD, class P>
+struct MarchSrc : ArraySrc<P> {
+    using ArraySrc<P>::ArraySrc;
+    static constexpr bool kAhead = false, kSlotwise = ORD == 4 && P::prec == BP_PREC_COMP16;
+};
+
 // Window shift: w[i] = w[i + 1].
 template <int N, class R>
 __device__ __forceinline__ void shift(R (&w)[N][4]) {
@@ -247,8 +257,8 @@ __global__ void __launch_bounds__(kMarchThreads, BP_MARCH_MINB) k_march(const Sh
                 V.s3[j] = dz_fwd<ORD, P>(wp, j, S);                    // p: D+z
             }
             if (act) {
-                if (P::prec == BP_PREC_COMP16 && r != (R)1) v_tail<2, ORD, P, !kLean, true>(S, c, x0, 0, z, r, mask, V);
-                else v_tail<2, ORD, P, !kLean, false>(S, c, x0, 0, z, r, mask, V);
+                if (P::prec == BP_PREC_COMP16 && r != (R)1) v_tail<2, ORD, P, !kLean, true>(S, c, x0, 0, z, r, mask, V, TailOut::v_of(S), MarchSrc<ORD, P>(S, c));
+                else v_tail<2, ORD, P, !kLean, false>(S, c, x0, 0, z, r, mask, V, TailOut::v_of(S), MarchSrc<ORD, P>(S, c));
             }
             shift(wp);
             shift(wzz);
@@ -333,8 +343,8 @@ __global__ void __launch_bounds__(kMarchThreads, BP_MARCH_MINB) k_march(const Sh
                 T.uxz[j] = dz_fwd<ORD, P>(wux, j, S);                   // vux: D+z
             }
             if (act) {
-                if (P::prec == BP_PREC_COMP16 && r != (R)1) t_tail<2, ORD, P, !kLean, true>(S, c, x0, 0, z, r, mask, T);
-                else t_tail<2, ORD, P, !kLean, false>(S, c, x0, 0, z, r, mask, T);
+                if (P::prec == BP_PREC_COMP16 && r != (R)1) t_tail<2, ORD, P, !kLean, true>(S, c, x0, 0, z, r, mask, T, TailOut::t_of(S), MarchSrc<ORD, P>(S, c));
+                else t_tail<2, ORD, P, !kLean, false>(S, c, x0, 0, z, r, mask, T, TailOut::t_of(S), MarchSrc<ORD, P>(S, c));
             }
             shift(wux);
             shift(wuz);

@@ -129,12 +129,14 @@ __host__ __device__ constexpr bool read_only_loads() {
 // warp's shared-memory slots, which asynchronous copies have filled.
 // span: cells x0 - HW .. x0 + 3 + HW of the chunk's row; rows: the chunk's cells
 // in rows -HW .. HW along y (AX 1) or z (AX 2); own: the chunk's cells.
-template <int ORD, class P, bool NC>
-struct GlobalSrc {
+template <int ORD, class P, bool NC, bool AHEAD = true>
+struct GlobalSrc : SrcForm {
+    static constexpr bool kAhead = AHEAD;
     using R = typename P::real;
     const ShotDesc& S;
     cidx c;
     int x0;
+    __device__ __forceinline__ GlobalSrc(const ShotDesc& S_, cidx c_, int x0_) : S(S_), c(c_), x0(x0_) {}
     template <int F>
     __device__ __forceinline__ void span(R (&v)[4 + ORD]) const {
         load_span<ORD, P, NC>(S.f[F], S.flo[F], c - x0, x0, S.nx, v);
@@ -656,7 +658,12 @@ __device__ __forceinline__ void chunk_unit(const ShotDesc& S, int x0, int y, int
     // an indexed medium's tuple indices first: their load overlaps the field loads
     unsigned ids = 0;
     if (med_on<P>(S)) ids = med_ids(S, c);
-    const GlobalSrc<ORD, P, NC> src{S, c, x0};
+    // The interleaved kernel holds both phases in one function and spills in 2D
+    // with the coefficients loaded ahead (FP32, us per step ahead -> not: 4040 x
+    // 2040 layered 229 -> 206, per-cell 257 -> 243, 817 x 1073 32.8 -> 31.7; the
+    // reference's rounding 232 -> 224, but 253 -> 261 per-cell, 41 -> 44: ahead).
+    constexpr bool AHEAD = NCOK || DIM == 3 || P::exact;
+    const GlobalSrc<ORD, P, NC, AHEAD> src(S, c, x0);
     chunk_work<DIM, ORD, P, VPHASE, NC, grouped<DIM, P, VPHASE>()>(S, src, c, x0, y, z, r, mask, ids, it, post);
 }
 
