@@ -18,6 +18,7 @@ struct Runner {
     long long ntiles = 0, ntiles_s = 0, ntiles_m = 0;
     int max_rec = 0;
     int grid_v = 1, grid_t = 1, grid_s = 1;
+    int sms = 148;                     // of the device (configure)
     bool staged = false;
     bool march = false;
     cudaStream_t st = nullptr;
@@ -51,11 +52,11 @@ struct Runner {
                    long long tiles_m, int maxrec, cudaStream_t s, int ctas_per_sm, int steps_per_graph) {
         prec = prec_; dim = dim_; order = order_;
         d_shots = d; nshots = n; ntiles = tiles; ntiles_s = tiles_s; ntiles_m = tiles_m; max_rec = maxrec; st = s;
-        int dev = 0, sms = 148;
+        int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int ov = phase_occupancy(prec, dim, order, true, rounding, indexed_form()),
-            ot = phase_occupancy(prec, dim, order, false, rounding, indexed_form());
+        int ov = phase_occupancy(prec, dim, order, true, rounding, dense_form()),
+            ot = phase_occupancy(prec, dim, order, false, rounding, dense_form());
         if (ctas_per_sm > 0) { ov = ov < ctas_per_sm ? ov : ctas_per_sm; ot = ot < ctas_per_sm ? ot : ctas_per_sm; }
         long long gv = (long long)ov * sms, gt = (long long)ot * sms;
         grid_v = (int)(gv < tiles ? gv : (tiles > 0 ? tiles : 1));
@@ -117,12 +118,17 @@ struct Runner {
 #endif
         return post_in_t && !march && !staged;
     }
-    // Whether the phases run as for an indexed medium.  2D order-2 COMP16 launches
-    // of per-cell media take their own shape (AsyncShape, step_async.cu) from 8
-    // tiles a CTA on: 4040 x 2040 262 -> 235 us per step, 817 x 1073 30.7 -> 32.9;
-    // order 4 loses by it (292 -> 358)
-    bool indexed_form() const {
-        return all_indexed || (prec == BP_PREC_COMP16 && !(dim == 2 && order == 2 && ntiles >= 8LL * 3 * 148));
+    // Whether the phases take the COMP16 shape for per-cell media (AsyncShape,
+    // step_async.cu): single 2D order-2 shots from 8 tiles for each CTA of the
+    // other shape (3 per SM) on.  us per step, B200, the other shape -> this one,
+    // per-cell media: 1907^2 (8 tiles a CTA) 128.7 -> 116.4, 2132^2 155 -> 137,
+    // 4040 x 2040 262 -> 235; below the line it changes sides with the last wave
+    // (740^2 25.6 -> 22.8, 1040^2 35.3 -> 38.2, 1349^2 74.1 -> 71.5, 1652^2 100.8 ->
+    // 88.6).  Order 4 loses by it (292 -> 358), and so do batches, which read the
+    // descriptor from shared memory (four shots of 15 M cells 564 -> 620).
+    bool dense_form() const {
+        return prec == BP_PREC_COMP16 && dim == 2 && order == 2 && !all_indexed && one && nshots == 1 && !multi_unit &&
+               ntiles >= 8LL * 3 * sms;
     }
     // launches of one step of the two-phase kernels
     int launches_per_step() const { return fused_post() ? 2 : 3; }
@@ -130,7 +136,7 @@ struct Runner {
         if (march) return launch_phase_march(prec, order, v, d_shots, nshots, ntiles_m, k, st);
         if (staged) return launch_phase_staged(prec, order, v, d_shots, nshots, ntiles_s, k, grid_s, d_err, st);
         return launch_phase(prec, dim, order, v, d_shots, nshots, ntiles, k, v ? grid_v : grid_t, st,
-                            (!v && fused_post()) ? 1 : 0, rounding, multi_unit, graded, indexed_form(), one);
+                            (!v && fused_post()) ? 1 : 0, rounding, multi_unit, graded, all_indexed, dense_form(), one);
     }
 
     // One step (index k of the chunk) of the two-phase kernels, or of the

@@ -16,10 +16,12 @@ namespace bpk {
 // sample (every receiver and the source lie in cells the T phase visits)
 // rounding = BP_ROUND_REFERENCE (FP32): the PolF32R instantiation; multi: the
 // tile shape has more (row, segment) units than a CTA has warps; indexed: every
-// shot reads an indexed medium; one: the host copy of a single shot's descriptor
+// shot reads an indexed medium; dense: the COMP16 shape for per-cell media
+// (Runner::dense_form); one: the host copy of a single shot's descriptor
 cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDesc* d_shots, int nshots,
                          long long ntiles, int k, int grid, cudaStream_t st, int post = 0, int rounding = 0,
-                         bool multi = false, bool graded = false, bool indexed = false, const ShotDesc* one = nullptr);
+                         bool multi = false, bool graded = false, bool indexed = false, bool dense = false,
+                         const ShotDesc* one = nullptr);
 cudaError_t launch_post(int prec, const ShotDesc* d_shots, int nshots, int max_rec, int k, int do_record,
                         cudaStream_t st);
 cudaError_t launch_inject(int prec, const ShotDesc* d_shots, int nshots, int k, cudaStream_t st);
@@ -58,8 +60,8 @@ cudaError_t launch_inter(int prec, int dim, int order, int rounding, const ShotD
 int seg_cells();
 // COMP16 phase kernels (step_async.cu), behind launch_phase and phase_occupancy
 cudaError_t launch_phase_async(int dim, int order, bool v, const ShotDesc* d, int nshots, long long ntiles, int k,
-                               int grid, cudaStream_t st, int post, const ShotDesc* one, bool indexed);
-int phase_async_occupancy(int dim, int order, bool v, bool indexed);
+                               int grid, cudaStream_t st, int post, const ShotDesc* one, bool dense);
+int phase_async_occupancy(int dim, int order, bool v, bool dense);
 // TMA-staged 2D phase kernels (step_staged.cu)
 bool staged_supported(int prec, int dim);
 bool staged_default();           // whether BP_KERNEL_AUTO picks the staged kernels where supported
@@ -67,7 +69,7 @@ int staged_tile_rows();
 int staged_tile_width();
 cudaError_t launch_phase_staged(int prec, int order, bool vphase, const ShotDesc* d, int nshots, long long ntiles,
                                 int k, int grid, int* err, cudaStream_t st);
-int phase_occupancy(int prec, int dim, int order, bool vphase, int rounding = 0, bool indexed = true);
+int phase_occupancy(int prec, int dim, int order, bool vphase, int rounding = 0, bool dense = false);
 // register-window marching 2D phase kernels (step_march.cu)
 bool march_supported(int prec, int dim);
 bool march_default();            // whether BP_KERNEL_AUTO picks the marching kernels where supported

@@ -301,7 +301,7 @@ static cudaError_t launch_ahead(bool v, const ShotDesc* d, int n, long long ntil
 }
 cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDesc* d_shots, int nshots,
                          long long ntiles, int k, int grid, cudaStream_t st, int post, int rounding, bool multi,
-                         bool graded, bool indexed, const ShotDesc* one) {
+                         bool graded, bool indexed, bool dense, const ShotDesc* one) {
     if (nshots != 1 || multi) one = nullptr;
     if (graded) {
         if (prec != BP_PREC_FP32 || rounding != BP_ROUND_FAST || order != 2) return cudaErrorInvalidValue;
@@ -323,7 +323,7 @@ cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDe
         return one && dim == 3 ? launch_one<PolF32>(dim, order, vphase, *one, (int)ntiles, k, grid, st, post)
                    : Launch<PolF32>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
     if (prec == BP_PREC_COMP16 && c16_async(dim, order))
-        return launch_phase_async(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, one, indexed);
+        return launch_phase_async(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, one, dense);
     if (prec == BP_PREC_COMP16)
         return one ? launch_one<PolC16>(dim, order, vphase, *one, (int)ntiles, k, grid, st, post)
                    : Launch<PolC16>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
@@ -375,7 +375,7 @@ cudaError_t launch_field_f64(int prec, const ShotDesc* d_shots, int f, double* o
     return cudaGetLastError();
 }
 
-int phase_occupancy(int prec, int dim, int order, bool vphase, int rounding, bool indexed) {
+int phase_occupancy(int prec, int dim, int order, bool vphase, int rounding, bool dense) {
     int n = 0;
     const void* fn = nullptr;
 #define BPK_FN(PP, D, O)                                                                   \
@@ -384,7 +384,7 @@ int phase_occupancy(int prec, int dim, int order, bool vphase, int rounding, boo
     if (prec == BP_PREC_FP32 && rounding == BP_ROUND_REFERENCE) {
         BPK_FN(PolF32R, 2, 2) BPK_FN(PolF32R, 2, 4) BPK_FN(PolF32R, 3, 2) BPK_FN(PolF32R, 3, 4)
     } else if (prec == BP_PREC_FP32) { BPK_FN(PolF32, 2, 2) BPK_FN(PolF32, 2, 4) BPK_FN(PolF32, 3, 2) BPK_FN(PolF32, 3, 4) }
-    else if (prec == BP_PREC_COMP16 && c16_async(dim, order)) return phase_async_occupancy(dim, order, vphase, indexed);
+    else if (prec == BP_PREC_COMP16 && c16_async(dim, order)) return phase_async_occupancy(dim, order, vphase, dense);
     else if (prec == BP_PREC_COMP16) { BPK_FN(PolC16, 3, 4) }
     else if (prec == BP_PREC_CBF16) { BPK_FN(PolB24, 2, 2) BPK_FN(PolB24, 2, 4) BPK_FN(PolB24, 3, 2) BPK_FN(PolB24, 3, 4) }
     else { BPK_FN(PolF64, 2, 2) BPK_FN(PolF64, 2, 4) BPK_FN(PolF64, 3, 2) BPK_FN(PolF64, 3, 4) }

@@ -21,8 +21,8 @@ namespace bpk {
 // 280 and more); 817 x 1073 41.5 -> 34.2; 296 x 296 x 232 uniform 2075 -> 1287 (3
 // CTAs: 2640), per-cell medium 2545 -> 1940; 140 x 130 x 120 228 -> 172.  With the
 // descriptor as a parameter and the four-value codec: 177, 227, 27, 980, 1620 and
-// 152.  Large 2D order-2 launches of per-cell media wait on their coefficients and
-// take 32 warps (DENSE, indexed_form in runner.h; indexed media 177 -> 181 by it).  Taking the chunk
+// 152.  Large 2D order-2 shots of per-cell media wait on their coefficients and
+// take 32 warps (DENSE, dense_form in runner.h; indexed media 177 -> 181 by it).  Taking the chunk
 // one output at a time (as the register tiles do in 3D) costs 10-35 % here, and
 // copies of the next unit under way while one is worked on cost occupancy: 50 %
 // slower.
@@ -65,12 +65,11 @@ __device__ __forceinline__ void async_units(const ShotDesc& S, char* mine, int l
     }
 }
 
-template <int DIM, int ORD, class P, bool VPHASE, bool DENSE>
-__global__ void __launch_bounds__(AsyncShape<DIM, ORD, P, VPHASE, DENSE>::NW * 32, (AsyncShape<DIM, ORD, P, VPHASE, DENSE>::MINB))
+template <int DIM, int ORD, class P, bool VPHASE>
+__global__ void __launch_bounds__(AsyncShape<DIM, ORD, P, VPHASE, false>::NW * 32, (AsyncShape<DIM, ORD, P, VPHASE, false>::MINB))
     k_phase_async(const ShotDesc* __restrict__ shots, int nshots, long long ntiles, int k, int post) {
     using R = typename P::real;
-    using C = AsyncShape<DIM, ORD, P, VPHASE, DENSE>;
-    using Src = typename C::Src;
+    using Src = typename AsyncShape<DIM, ORD, P, VPHASE, false>::Src;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ ShotDesc sdesc;
     extern __shared__ __align__(16) char slots[];
@@ -93,7 +92,7 @@ __global__ void __launch_bounds__(AsyncShape<DIM, ORD, P, VPHASE, DENSE>::NW * 3
             cur = si;
             it = *sdesc.step_base + k;
             live = !sdesc.done && it < sdesc.nt;
-            if constexpr (P::prec == BP_PREC_COMP16) r = live ? sdesc.rtab[it] : 1.0f;
+            r = live ? sdesc.rtab[it] : 1.0f;
         }
         if (!live) continue;
         const ShotDesc& S = sdesc;
@@ -110,8 +109,7 @@ __global__ void __launch_bounds__(AsyncShape<DIM, ORD, P, VPHASE, DENSE>::NW * 3
     extern __shared__ __align__(16) char slots[];
     const int it = *S.step_base + k;
     if (S.done || it >= S.nt) return;
-    R r = (R)1;
-    if constexpr (P::prec == BP_PREC_COMP16) r = S.rtab[it];
+    const R r = S.rtab[it];
     const int G = gridDim.x;
     const bool back = !VPHASE && ntiles > G;
     const int t0 = back ? blockIdx.x + (ntiles - 1 - (int)blockIdx.x) / G * G : blockIdx.x;
@@ -122,56 +120,66 @@ __global__ void __launch_bounds__(AsyncShape<DIM, ORD, P, VPHASE, DENSE>::NW * 3
 
 // The kernels use more dynamic shared memory than a launch may without this
 // (set per device, so before every launch that is not a graph replay).
-template <int D, int O, class P, bool V, bool DN>
-static cudaError_t allow_smem() {
-    cudaError_t e = cudaFuncSetAttribute(k_phase_async_one<D, O, P, V, DN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         AsyncShape<D, O, P, V, DN>::kSmem);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_phase_async<D, O, P, V, DN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                AsyncShape<D, O, P, V, DN>::kSmem);
+template <class K>
+static cudaError_t allow_smem(K kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
-template <int D, int O, class P, bool V, bool DN>
-static cudaError_t launch_a(const ShotDesc* d, int nshots, long long ntiles, int k, int grid, cudaStream_t st, int post,
-                            const ShotDesc* one) {
+template <int D, int O, class P, bool V, bool DN = false>
+static cudaError_t launch_single(const ShotDesc& S, long long ntiles, int k, int grid, cudaStream_t st, int post) {
     using C = AsyncShape<D, O, P, V, DN>;
-    cudaError_t e = allow_smem<D, O, P, V, DN>();
+    cudaError_t e = allow_smem(k_phase_async_one<D, O, P, V, DN>, C::kSmem);
     if (e != cudaSuccess) return e;
-    if (one) k_phase_async_one<D, O, P, V, DN><<<grid, C::NW * 32, C::kSmem, st>>>(*one, (int)ntiles, k, post);
-    else k_phase_async<D, O, P, V, DN><<<grid, C::NW * 32, C::kSmem, st>>>(d, nshots, ntiles, k, post);
+    k_phase_async_one<D, O, P, V, DN><<<grid, C::NW * 32, C::kSmem, st>>>(S, (int)ntiles, k, post);
     return cudaGetLastError();
 }
-template <int D, int O, class P, bool V, bool DN>
-static int occupancy_a() {
+template <int D, int O, class P, bool V>
+static cudaError_t launch_table(const ShotDesc* d, int nshots, long long ntiles, int k, int grid, cudaStream_t st, int post) {
+    using C = AsyncShape<D, O, P, V, false>;
+    cudaError_t e = allow_smem(k_phase_async<D, O, P, V>, C::kSmem);
+    if (e != cudaSuccess) return e;
+    k_phase_async<D, O, P, V><<<grid, C::NW * 32, C::kSmem, st>>>(d, nshots, ntiles, k, post);
+    return cudaGetLastError();
+}
+template <class K>
+static int occupancy_a(K kernel, int threads, int bytes) {
     int n = 0;
-    if (allow_smem<D, O, P, V, DN>() != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_phase_async<D, O, P, V, DN>, AsyncShape<D, O, P, V, DN>::NW * 32,
-                                                      AsyncShape<D, O, P, V, DN>::kSmem) != cudaSuccess)
+    if (allow_smem(kernel, bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, bytes) != cudaSuccess)
         return 1;
     return n > 0 ? n : 1;
 }
 
 #define BPK_EACH(X) X(2, 2) X(2, 4) X(3, 2)
+// dense: the shape for per-cell media, 2D order-2 single shots only
 cudaError_t launch_phase_async(int dim, int order, bool v, const ShotDesc* d, int nshots, long long ntiles, int k,
-                               int grid, cudaStream_t st, int post, const ShotDesc* one, bool indexed) {
+                               int grid, cudaStream_t st, int post, const ShotDesc* one, bool dense) {
+    if (dense) {
+        if (dim != 2 || order != 2 || !one) return cudaErrorInvalidValue;
+        return v ? launch_single<2, 2, PolC16, true, true>(*one, ntiles, k, grid, st, 0)
+                 : launch_single<2, 2, PolC16, false, true>(*one, ntiles, k, grid, st, post);
+    }
 #define BPK_LAUNCH(D, O)                                                                                            \
     if (dim == D && order == O) {                                                                                   \
-        if (D == 2 && O == 2 && !indexed)                                                                                     \
-            return v ? launch_a<D, O, PolC16, true, D == 2 && O == 2>(d, nshots, ntiles, k, grid, st, 0, one)                 \
-                     : launch_a<D, O, PolC16, false, D == 2 && O == 2>(d, nshots, ntiles, k, grid, st, post, one);            \
-        return v ? launch_a<D, O, PolC16, true, false>(d, nshots, ntiles, k, grid, st, 0, one)                      \
-                 : launch_a<D, O, PolC16, false, false>(d, nshots, ntiles, k, grid, st, post, one);                 \
+        if (one) return v ? launch_single<D, O, PolC16, true>(*one, ntiles, k, grid, st, 0)                         \
+                          : launch_single<D, O, PolC16, false>(*one, ntiles, k, grid, st, post);                    \
+        return v ? launch_table<D, O, PolC16, true>(d, nshots, ntiles, k, grid, st, 0)                              \
+                 : launch_table<D, O, PolC16, false>(d, nshots, ntiles, k, grid, st, post);                         \
     }
     BPK_EACH(BPK_LAUNCH)
 #undef BPK_LAUNCH
     return cudaErrorInvalidValue;
 }
-int phase_async_occupancy(int dim, int order, bool v, bool indexed) {
-#define BPK_OCC(D, O)                                                                                               \
-    if (dim == D && order == O) {                                                                                   \
-        if (D == 2 && O == 2 && !indexed)                                                                                     \
-            return v ? occupancy_a<D, O, PolC16, true, D == 2 && O == 2>() : occupancy_a<D, O, PolC16, false, D == 2 && O == 2>();      \
-        return v ? occupancy_a<D, O, PolC16, true, false>() : occupancy_a<D, O, PolC16, false, false>();            \
-    }
-    BPK_EACH(BPK_OCC)
+int phase_async_occupancy(int dim, int order, bool v, bool dense) {
+#define BPK_OCC(KERNEL, D, O, V, DN) occupancy_a(KERNEL, AsyncShape<D, O, PolC16, V, DN>::NW * 32, AsyncShape<D, O, PolC16, V, DN>::kSmem)
+    if (dense && dim == 2 && order == 2)
+        return v ? BPK_OCC((k_phase_async_one<2, 2, PolC16, true, true>), 2, 2, true, true)
+                 : BPK_OCC((k_phase_async_one<2, 2, PolC16, false, true>), 2, 2, false, true);
+#define BPK_EACH_OCC(D, O)                                                                                          \
+    if (dim == D && order == O)                                                                                     \
+        return v ? BPK_OCC((k_phase_async<D, O, PolC16, true>), D, O, true, false)                                  \
+                 : BPK_OCC((k_phase_async<D, O, PolC16, false>), D, O, false, false);
+    BPK_EACH(BPK_EACH_OCC)
+#undef BPK_EACH_OCC
 #undef BPK_OCC
     return 1;
 }
