@@ -138,7 +138,7 @@ static std::vector<TileShape> shape_candidates(int dim, int prec) {
 int BatchCore::autotune(int budget_steps) {
     if (shots.empty()) return BP_OK;
     long long cells = total_cells();
-    TuneKey key{dim, order, prec + 16 * rounding, (int)std::floor(std::log2((double)std::max(cells, 1LL))),
+    TuneKey key{dim, order, prec + 16 * rounding, run.all_indexed, (int)std::floor(std::log2((double)std::max(cells, 1LL))),
                 (int)std::floor(std::log2((double)shots.size()))};
     const bool fix_shape = shape.rows > 0, fix_c = ctas_per_sm > 0, fix_s = steps_per_sync > 0;
     const bool fix_k = kernel != BP_KERNEL_AUTO;

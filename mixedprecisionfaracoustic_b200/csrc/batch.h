@@ -11,10 +11,12 @@
 namespace bpk {
 
 struct TuneKey {
-    int dim, order, prec, cells_class, shots_class;   // log2 of the total cells and of the shot count
+    int dim, order, prec;
+    bool indexed;                        // every shot reads an indexed medium (selects kernels, Runner::all_indexed)
+    int cells_class, shots_class;        // log2 of the total cells and of the shot count
     bool operator<(const TuneKey& o) const {
-        return std::tie(dim, order, prec, cells_class, shots_class) <
-               std::tie(o.dim, o.order, o.prec, o.cells_class, o.shots_class);
+        return std::tie(dim, order, prec, indexed, cells_class, shots_class) <
+               std::tie(o.dim, o.order, o.prec, o.indexed, o.cells_class, o.shots_class);
     }
 };
 struct TuneVal {
@@ -24,7 +26,7 @@ struct TuneVal {
 };
 
 // Process-wide cache of autotuning results keyed by (dim, order, precision
-// and rounding, grid class: log2 of the batch's cells and of its shot count).
+// and rounding, medium form, grid class: log2 of the batch's cells and of its shot count).
 std::map<TuneKey, TuneVal>& tune_cache();
 
 struct BatchCore {

@@ -14,14 +14,13 @@ pytestmark = pytest.mark.gpu
 
 FAMILIES = {"fused": ("fp32", "comp16", "cbf16"), "march": ("fp32", "comp16"),
             "interleaved": ("fp32", "comp16", "cbf16", "fp64")}
+# the marching kernels read the per-cell arrays only
+CASES = [(f, p, m) for f, ps in FAMILIES.items() for p in ps for m in ("dense", "auto") if (f, m) != ("march", "auto")]
 
 
-@pytest.mark.parametrize("medium", ["dense", "auto"])
 @pytest.mark.parametrize("order", [2, 4])
-@pytest.mark.parametrize("family,prec", [(f, p) for f, ps in FAMILIES.items() for p in ps])
+@pytest.mark.parametrize("family,prec,medium", CASES)
 def test_family_equals_the_register_kernels(family, prec, order, medium):
-    if family == "march" and medium == "auto":
-        pytest.skip("the marching kernels read the per-cell arrays only")
     cfg, med = config1(precision=prec, nx=277, nz=101, nt=223, npml=9, order=order, nrec=32)
     cfg.medium = medium
     ref_tr, ref_f = run(cfg, med, "register", [cfg.nt])
