@@ -241,10 +241,12 @@ static cudaError_t launch_one(int dim, int order, bool v, const ShotDesc& S, int
         else k_phase_one<D, O, P, false, PF><<<grid, kThreads, 0, st>>>(S, ntiles, k, post);                  \
         return cudaGetLastError();                                                                            \
     }
-    if constexpr (P::graded) {
+    if constexpr (std::is_same_v<P, PolF32>) {     // 2D only with the prefetch, 3D order 4 only without
+        BPK_ONE(3, 2)
+        if constexpr (PF) { BPK_ONE(2, 2) BPK_ONE(2, 4) }
+        else { BPK_ONE(3, 4) }
+    } else if constexpr (P::graded) {
         BPK_ONE(2, 2) BPK_ONE(3, 2)
-    } else if constexpr (P::prec == BP_PREC_COMP16) {
-        BPK_ONE(3, 4)
     } else {
         BPK_ONE(2, 2) BPK_ONE(2, 4) BPK_ONE(3, 2) BPK_ONE(3, 4)
     }
@@ -324,9 +326,11 @@ cudaError_t launch_phase(int prec, int dim, int order, bool vphase, const ShotDe
                    : Launch<PolF32>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
     if (prec == BP_PREC_COMP16 && c16_async(dim, order))
         return launch_phase_async(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, one, dense);
+    // 3D order 4: the V phase spills 200 bytes with the descriptor as a parameter
+    // and none without, for the same time (us per step, 296 x 296 x 232 uniform 2630
+    // and 2600, per-cell 3053 and 3057; 200 x 190 x 180 787 and 788)
     if (prec == BP_PREC_COMP16)
-        return one ? launch_one<PolC16>(dim, order, vphase, *one, (int)ntiles, k, grid, st, post)
-                   : Launch<PolC16>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
+        return Launch<PolC16>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
     if (prec == BP_PREC_CBF16)
         return one ? launch_one<PolB24>(dim, order, vphase, *one, (int)ntiles, k, grid, st, post)
                    : Launch<PolB24>::phase(dim, order, vphase, d_shots, nshots, ntiles, k, grid, st, post, multi);
