@@ -270,9 +270,12 @@ __device__ __forceinline__ void t_chunk(const ShotDesc& S, const Src& src, cidx 
 // = T).  Measured on B200 (3D: 192^3 and 552 x 552 x 424 order 2, 200^3
 // order 4; 2D: 4040 x 2040 order 2): 3D COMP16 both (12-16 % off the step,
 // its spills gone); 2D COMP16 the T phase (13 % off it, the V phase 2 %
-// slower grouped); FP64 the 3D T phase (with 2 CTAs per SM, 25-30 % off the
-// 3D step); FP32 neither (10-20 % slower, its latency-bound phases losing the
-// loads they had in flight).
+// slower grouped); FP64 both in 3D: the T phase with 2 CTAs per SM 25-30 % off
+// the 3D step, the V phase, which spills 516-860 bytes as a whole chunk (an axis'
+// memory variables at once) and none grouped, us per step 140 x 130 x 120 345 ->
+// 312, order 4 366 -> 334, 200 x 190 x 180 905 -> 825, 296 x 296 x 232 2760 -> 2536,
+// order 4 3295 -> 3000; FP32 neither (10-20 % slower, its latency-bound phases
+// losing the loads they had in flight).
 #ifndef BP_GROUP3_C16
 #define BP_GROUP3_C16 3
 #endif
@@ -280,7 +283,7 @@ __device__ __forceinline__ void t_chunk(const ShotDesc& S, const Src& src, cidx 
 #define BP_GROUP3_F32 0
 #endif
 #ifndef BP_GROUP3_F64
-#define BP_GROUP3_F64 2
+#define BP_GROUP3_F64 3
 #endif
 #ifndef BP_GROUP2_C16
 #define BP_GROUP2_C16 2
@@ -653,7 +656,10 @@ __device__ __forceinline__ void chunk_unit(const ShotDesc& S, int x0, int y, int
     if (!row_updated<DIM, ORD>(S, y, z)) return;
     const unsigned mask = chunk_mask<ORD>(S, x0);
     if (!mask) return;
-    constexpr bool NC = read_only_loads<DIM, P, VPHASE>() && NCOK && !grouped<DIM, P, VPHASE>();
+    // the interleaved kernel's FP64 V phase, at one CTA per SM, takes whole chunks
+    // (200 x 190 x 180 1649 us per step, 1829 grouped; order 4 1698 and 1855)
+    constexpr bool GROUPED = grouped<DIM, P, VPHASE>() && (NCOK || !VPHASE || P::prec != BP_PREC_FP64);
+    constexpr bool NC = read_only_loads<DIM, P, VPHASE>() && NCOK && !GROUPED;
     const cidx c = x0 + y * S.pitch + z * (cidx)S.plane;
     // an indexed medium's tuple indices first: their load overlaps the field loads
     unsigned ids = 0;
@@ -664,7 +670,7 @@ __device__ __forceinline__ void chunk_unit(const ShotDesc& S, int x0, int y, int
     // reference's rounding 232 -> 224, but 253 -> 261 per-cell, 41 -> 44: ahead).
     constexpr bool AHEAD = NCOK || DIM == 3 || P::exact;
     const GlobalSrc<ORD, P, NC, AHEAD> src(S, c, x0);
-    chunk_work<DIM, ORD, P, VPHASE, NC, grouped<DIM, P, VPHASE>()>(S, src, c, x0, y, z, r, mask, ids, it, post);
+    chunk_work<DIM, ORD, P, VPHASE, NC, GROUPED>(S, src, c, x0, y, z, r, mask, ids, it, post);
 }
 
 // The (row, segment) units of tile (rb, sb) of shot S in one phase: the
