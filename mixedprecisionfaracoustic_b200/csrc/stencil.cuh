@@ -18,23 +18,27 @@ namespace bpk {
 // and the quotient is formed from the divisor's reciprocal y by two residual
 // corrections q += y (a - q b) with exact fused residuals (Markstein, IBM J.
 // Res. Dev. 34(1), 1990), which round correctly where nothing under- or
-// overflows.  A subnormal float result must not be rounded twice, so q is
-// first rounded to odd (Boldo and Melquiond, IEEE Trans. Comput. 57(4), 2008):
-// 24 bits to odd, then to at most 22 to nearest, is one rounding to nearest.
-// The binade below the smallest normal (23 bits) and quotients out of range
-// (infinite, NaN) take the division itself.  Equal to a / b bit for bit
+// overflows.  A subnormal result must not be rounded twice, so q is first
+// rounded to odd (Boldo and Melquiond, IEEE Trans. Comput. 57(4), 2008): 24 bits
+// to odd, then to at most 22 to nearest, is one rounding to nearest (FP64: 53
+// and 51).  The binade below the smallest normal (one bit more) and quotients
+// out of range (infinite, NaN) take the division itself.  Equal to a / b bit for bit
 // (tests/test_gpu_quotient.py).
 template <class R> struct QuotRange;
 template <> struct QuotRange<float> {
-    static constexpr float small = 0x1p-30f, up = 0x1p64f, down = 0x1p-64f, lo = 0x1p-61f, hi = 0x1p120f;
+    static constexpr float small = 0x1p-30f, up = 0x1p64f, down = 0x1p-64f, lo = 0x1p-61f, sub = 0x1p-63f, hi = 0x1p120f;
 };
 template <> struct QuotRange<double> {
-    static constexpr double small = 0x1p-300, up = 0x1p600, down = 0x1p-600, lo = 0x1p-420, hi = 0x1p1000;
+    static constexpr double small = 0x1p-300, up = 0x1p600, down = 0x1p-600, lo = 0x1p-420, sub = 0x1p-423, hi = 0x1p1000;
 };
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ int bits_of(float a) { return __float_as_int(a); }
+__device__ __forceinline__ long long bits_of(double a) { return __double_as_longlong(a); }
+__device__ __forceinline__ float of_bits(int a) { return __int_as_float(a); }
+__device__ __forceinline__ double of_bits(long long a) { return __longlong_as_double(a); }
 
 // a / b for y = 1 / b to within an ulp
 template <class R>
@@ -47,13 +51,11 @@ __device__ __forceinline__ R quot_y(R a, R b, R y) {
     q = fma_rn(fma_rn(-q, b, t), y, q);
     if (fabs(q) >= Q::lo && fabs(q) < Q::hi) return mul_rn(q, tiny ? Q::down : (R)1);
     if (a == (R)0) return mul_rn(a, b);            // the zero with the quotient's sign
-    if constexpr (sizeof(R) == 4) {
-        if (tiny && fabs(q) < 0x1p-63f) {
-            const float r = fma_rn(-q, b, t);      // a 2^64 - q b, exact
-            int w = __float_as_int(q);
-            if (r != 0.0f) w = (w + ((__float_as_int(r) ^ __float_as_int(b) ^ w) >> 31)) | 1;
-            return mul_rn(__int_as_float(w), Q::down);
-        }
+    if (tiny && fabs(q) < Q::sub) {
+        const R r = fma_rn(-q, b, t);              // a up - q b, exact
+        auto w = bits_of(q);
+        if (r != (R)0) w = (w + ((bits_of(r) ^ bits_of(b) ^ w) >> (8 * sizeof(R) - 1))) | 1;
+        return mul_rn(of_bits(w), Q::down);
     }
     return a / b;
 }
