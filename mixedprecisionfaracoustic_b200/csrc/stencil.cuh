@@ -74,7 +74,7 @@ __device__ __forceinline__ float recip(float b) {
 // 175), 165.1 with it (156, 175); order 4 201.7, 190.5 and 186.0; 817 x 1073 at
 // step 1500 24.0, 22.3 and 22.0.  In 3D CBF16 keeps the division: 200 x 190 x 180
 // 367 against 376 at step 600, 296 x 296 x 232 965 against 975 early, though 1208
-// against 1092 late.  So does FP64, whose exponents never run out.
+// against 1092 late.  So does FP64.
 // TEST0: FP32 tests for zero as well (SrcForm).
 template <class P, int DIM, bool TEST0 = false>
 __device__ __forceinline__ typename P::real quot(typename P::real a, typename P::real b) {

@@ -1,12 +1,12 @@
 // step.cu - the hot path: velocity phase, stress phase and post-step kernels.
 //
 // Reference kernels replaced (Zhitao-Zhang/MixedPrecisionFarAcoustic):
-//   FD_V   Float/main.cu:64-192,  Half/main.cu:156-268  -> k_vphase
-//   FD_T   Float/main.cu:194-295, Half/main.cu:270-371  -> k_tphase
+//   FD_V   Float/main.cu:64-192,  Half/main.cu:156-268  -> k_phase (VPHASE)
+//   FD_T   Float/main.cu:194-295, Half/main.cu:270-371  -> k_phase (T)
 //   Source Float/main.cu:45-59,   Half/main.cu:135-151  -> k_post (inject)
 //   trace capture Float/main.cu:1075-1093               -> k_post (record)
 //   ScaleHalfArray/ScaleCompressedArray Half/main.cu:102-114: folded into
-//   k_vphase/k_tphase as a per-step factor on every old state value.
+//   k_phase as a per-step factor on every old state value.
 //
 // Work decomposition: a tile is 8 rows x 128 cells of one shot; a CTA of 8
 // warps takes one tile at a time (one row per warp, 4 consecutive x cells per
@@ -26,7 +26,10 @@ namespace bpk {
 // 409 -> 403 (B200).  Everything else loses by it: per-cell media, whose
 // coefficients keep DRAM busy (4040 x 2040 196 -> 221, 424 x 424 x 328 2742 ->
 // 3392), the 3-byte and FP64 formats, which wait less on loads (COMP16 255 ->
-// 264, FP64 532 -> 614), and short launches (817 x 1073 19.2 -> 20.0).
+// 264, FP64 532 -> 614), and some short launches (817 x 1073 19.2 -> 20.0).  Around
+// the line, without -> with: 2D order 2 at 3, 6, 8, 10 and 14 tiles a CTA 33.7 -> 32.7,
+// 52.4 -> 51.5, 70.7 -> 67.6, 94.4 -> 89.5, 119.8 -> 113.0; 3D 73.1 -> 74.4, 119.7 ->
+// 118.8, 158.0 -> 158.6, 181.8 -> 174.5, 251.9 -> 245.2.
 constexpr int kAheadTiles = 8;
 template <int DIM, int ORD, class P, bool VPHASE, bool MU, bool PF = false>
 __global__ void __launch_bounds__(kThreads, (phase_min_blocks<DIM, ORD, P, VPHASE>())) k_phase(const ShotDesc* __restrict__ shots, int nshots,
@@ -90,8 +93,8 @@ __global__ void __launch_bounds__(kThreads, (phase_min_blocks<DIM, ORD, P, VPHAS
 // pointers and extents are constant-bank operands where k_phase loads them from
 // shared memory for every use, and a launch starts on its step counter instead
 // of on the descriptor.  Measured on B200, us per step, k_phase -> this: 4040 x
-// 2040 FP32 147.3 -> 144.3, order 4 155.7 -> 151.6, CBF16 171 -> 165, FP64 408 ->
-// 398; 3041 x 1547 order 4 CBF16 137 -> 129; 200^3 order 4 435 -> 427; 424 x 424 x
+// 2040 FP32 147.3 -> 144.3, order 4 155.7 -> 151.6, CBF16 186.4 -> 180.3 (over 8000
+// steps), FP64 408 -> 398; 3041 x 1547 order 4 CBF16 137 -> 129; 200^3 order 4 435 -> 427; 424 x 424 x
 // 328 2743 -> 2690; 192^3 reference rounding 404 -> 387.
 template <int DIM, int ORD, class P, bool VPHASE, bool PF>
 __global__ void __launch_bounds__(kThreads, (phase_min_blocks<DIM, ORD, P, VPHASE>()))

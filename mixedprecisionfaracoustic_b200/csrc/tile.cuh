@@ -20,7 +20,8 @@ constexpr int kSegCells = 128;
 // z planes, so the z neighbours of most rows are rows of the same tile (2D
 // tiles are 8 consecutive z rows).  Measured on B200 (192^3, 200^3 order 4,
 // 552 x 552 x 424; all shapes bit-identical): FP32 is fastest with 1 x 8
-// (up to 8 % over 8 x 1), COMP16 with 4 x 2.
+// (up to 8 % over 8 x 1), COMP16, in the register kernels that order 4 still
+// runs, with 4 x 2.
 __host__ __device__ constexpr int tile_tz(int prec) {
     return prec == BP_PREC_FP32 ? 8 : (prec == BP_PREC_COMP16 ? 2 : 1);
 }
@@ -41,18 +42,12 @@ __device__ __forceinline__ int locate_shot(const ShotDesc* shots, int nshots, lo
 #endif
 // Resident CTAs per SM the 2D phase kernels are register-limited to (1 = no
 // limit).  Measured on B200 for the 4040 x 2040 order-2 grid: FP32 is fastest
-// at 3 (80 registers, no spills); COMP16, whose decode/encode chains leave it
-// latency-bound, at 6 (40 registers) for both phases, the T phase in grouped
-// form (below), both with some spilled values; FP64 at 2 (128 registers;
-// uncapped it takes ~150, one CTA per SM, and runs 40 % slower).
+// at 3 (80 registers; the V phase spills 12-16 bytes, 40 in the form for tiles of
+// more units than warps); FP64 at 2 (128 registers; uncapped it takes ~150, one
+// CTA per SM, and runs 40 % slower).  2D COMP16 runs the staged kernels, whose
+// caps are in step_async.cu.
 #ifndef BP_MINB_F32
 #define BP_MINB_F32 3
-#endif
-#ifndef BP_MINB_C16
-#define BP_MINB_C16 6
-#endif
-#ifndef BP_MINB_C16_V
-#define BP_MINB_C16_V 6
 #endif
 #ifndef BP_MINB_F64
 #define BP_MINB_F64 2
@@ -91,8 +86,7 @@ template <int DIM, int ORD, class P, bool VPHASE>
 __host__ __device__ constexpr int phase_min_blocks() {
     if (P::store == BP_PREC_CBF16) return DIM == 3 ? BP_MINB3_B24 : (VPHASE ? BP_MINB_B24_V : BP_MINB_B24);
     if (DIM == 3) return P::prec == BP_PREC_FP32 ? BP_MINB3_F32 : P::prec == BP_PREC_COMP16 ? BP_MINB3_C16 : BP_MINB3_F64;
-    return P::prec == BP_PREC_FP32 ? BP_MINB_F32
-                                   : P::prec == BP_PREC_COMP16 ? (VPHASE ? BP_MINB_C16_V : BP_MINB_C16) : BP_MINB_F64;
+    return P::prec == BP_PREC_FP32 ? BP_MINB_F32 : BP_MINB_F64;
 }
 // How a tile learns its step index: 1 = once per shot per launch, 0 = a read
 // of the step counter per tile (measured faster for FP32 at 80 registers).
@@ -269,8 +263,8 @@ __device__ __forceinline__ void t_chunk(const ShotDesc& S, const Src& src, cidx 
 // Which phases take this form, per dimension and precision (bit 0 = V, bit 1
 // = T).  Measured on B200 (3D: 192^3 and 552 x 552 x 424 order 2, 200^3
 // order 4; 2D: 4040 x 2040 order 2): 3D COMP16 both (12-16 % off the step,
-// its spills gone); 2D COMP16 the T phase (13 % off it, the V phase 2 %
-// slower grouped); FP64 both in 3D: the T phase with 2 CTAs per SM 25-30 % off
+// its spills gone); 2D COMP16, here the interleaved kernel alone, the T phase (13 %
+// off it, the V phase 2 % slower grouped); FP64 both in 3D: the T phase with 2 CTAs per SM 25-30 % off
 // the 3D step, the V phase, which spills 516-860 bytes as a whole chunk (an axis'
 // memory variables at once) and none grouped, us per step 140 x 130 x 120 345 ->
 // 312, order 4 366 -> 334, 200 x 190 x 180 905 -> 825, 296 x 296 x 232 2760 -> 2536,
@@ -701,7 +695,7 @@ __device__ __forceinline__ void tile_units(const ShotDesc& S, int rb, int sb, in
     };
     // MU: tiles of more units than warps (16-row or 8 x 2 tiles); the
     // one-unit form keeps no loop state live across the chunk code, which
-    // costs the 2D FP32 V phase its spill-free 80 registers otherwise
+    // spills more of the 2D FP32 V phase's 80 registers
     if constexpr (MU) {
         for (int u = warp; u < units; u += kWarps) unit(u);
     } else {
